@@ -147,6 +147,17 @@ __device__ __forceinline__ long long warp_incl_scan(long long v) {
   return v;
 }
 
+// Inclusive warp scan (int)
+__device__ __forceinline__ int warp_incl_scan_i32(int v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(VK_FULL, v, o);
+    if (lane >= o) v += t;
+  }
+  return v;
+}
+
 __device__ __forceinline__ long long warp_sum(long long v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(VK_FULL, v, o);

@@ -298,17 +298,29 @@ k1_brute_k(int64_t n, const int32_t* c_hyp, const int32_t* c_row, const int32_t*
 }
 
 // ------------------------------------------------------------------------------------------ K2
-template <bool SHIFT>
-__global__ void __launch_bounds__(vk::K2_WARPS * 32)
+__global__ void __launch_bounds__(vk::KD_WARPS * 32, vk::KD_CTAS)
 k2_compat_k(int n_spec, const int64_t* cand_off, const int32_t* c_row, const int8_t* c_maxfz, const int32_t* spec_ids,
             const int64_t* pk_off, const float* pk_mass, const float* pk_int, const int64_t* seq_off,
             const uint8_t* len, const uint64_t* mask, const float* mass32, const uint8_t* res, float tol_lo,
-            float tol_hi, const float* c_shift, vk::K2Out out) {
+            float tol_hi, vk::K2Out out) {
+  __shared__ vk::SmemFrag sf;
+  __shared__ vk::K2DenseSmem S;
+  frag_from_const(sf);
+  __syncthreads();
+  vk::k2_dense_body(S, sf, n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off, pk_mass, pk_int, seq_off, len, mask,
+                    mass32, res, tol_lo, tol_hi, out);
+}
+
+__global__ void __launch_bounds__(vk::K2_WARPS * 32)
+k2_compat_shift_k(int n_spec, const int64_t* cand_off, const int32_t* c_row, const int8_t* c_maxfz,
+                  const int32_t* spec_ids, const int64_t* pk_off, const float* pk_mass, const float* pk_int,
+                  const int64_t* seq_off, const uint8_t* len, const uint64_t* mask, const float* mass32,
+                  const uint8_t* res, float tol_lo, float tol_hi, const float* c_shift, vk::K2Out out) {
   __shared__ vk::SmemFrag sf;
   frag_from_const(sf);
   __syncthreads();
-  vk::k2_body<SHIFT>(sf, n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off, pk_mass, pk_int, seq_off, len, mask,
-                     mass32, res, tol_lo, tol_hi, c_shift, out);
+  vk::k2_body(sf, n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off, pk_mass, pk_int, seq_off, len, mask, mass32, res,
+              tol_lo, tol_hi, c_shift, out);
 }
 
 int k2_compat(int n_spec, const int64_t* cand_off, const int32_t* c_row, const int8_t* c_maxfz,
@@ -319,16 +331,19 @@ int k2_compat(int n_spec, const int64_t* cand_off, const int32_t* c_row, const i
               void* stream) {
   if (n_spec <= 0) return 0;
   vk::K2Out out{o_hs, o_sb, o_sy, o_ppm, o_mb, o_my, o_lb, o_ly};
-  const unsigned grid = (unsigned)((n_spec + vk::K2_WARPS - 1) / vk::K2_WARPS);
   cudaStream_t st = (cudaStream_t)stream;
-  if (c_shift)
-    k2_compat_k<true><<<grid, vk::K2_WARPS * 32, 0, st>>>(n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off,
-                                                           pk_mass, pk_int, seq_off, len, mask, mass32, res, tol_lo,
-                                                           tol_hi, c_shift, out);
-  else
-    k2_compat_k<false><<<grid, vk::K2_WARPS * 32, 0, st>>>(n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off,
-                                                            pk_mass, pk_int, seq_off, len, mask, mass32, res, tol_lo,
-                                                            tol_hi, nullptr, out);
+  if (c_shift) {
+    const unsigned grid = (unsigned)((n_spec + vk::K2_WARPS - 1) / vk::K2_WARPS);
+    k2_compat_shift_k<<<grid, vk::K2_WARPS * 32, 0, st>>>(n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off, pk_mass,
+                                                          pk_int, seq_off, len, mask, mass32, res, tol_lo, tol_hi,
+                                                          c_shift, out);
+    return vk_launch_status();
+  }
+  int err = 0;
+  const int grid = vk::k2_dense_grid(k2_compat_k, n_spec, &err);
+  if (err) return err;
+  k2_compat_k<<<grid, vk::KD_WARPS * 32, 0, st>>>(n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off, pk_mass, pk_int,
+                                                  seq_off, len, mask, mass32, res, tol_lo, tol_hi, out);
   return vk_launch_status();
 }
 
@@ -415,7 +430,7 @@ int vk_k2(int n_spec, const int64_t* cand_off, const int32_t* c_row, const int8_
           const uint8_t* len, const uint64_t* mask, const float* mass32, const uint8_t* res, float tol_lo,
           float tol_hi, double* o_hs, float* o_sb, float* o_sy, float* o_ppm, int16_t* o_mb, int16_t* o_my,
           int16_t* o_lb, int16_t* o_ly, int threads, void* stream) {
-  (void)threads;   // the launch shape is this library's (one warp per spectrum)
+  (void)threads;   // the launch shape is this library's
   return k2_compat(n_spec, cand_off, c_row, c_maxfz, spec_ids, pk_off, pk_mass, pk_int, seq_off, len, mask, mass32,
                    res, tol_lo, tol_hi, nullptr, o_hs, o_sb, o_sy, o_ppm, o_mb, o_my, o_lb, o_ly, stream);
 }

@@ -380,8 +380,9 @@ __global__ void __launch_bounds__(FS_MAX_WARPS * 32) fused_search_k(FusedParams 
       const float span = np > 0 ? __fsub_rn(sm[np - 1], pt.m0) : 0.f;
       pt.inv_w = span > 0.f ? __fdiv_rn((float)vk::K2_BUCKETS, span) : 0.f;
       for (int j = threadIdx.x; j < n_cand; j += blockDim.x)
-        vk::k2_score<false>(fp, pt, frow[j], h_mfz[fhl[j]], P.seq_off, P.len, P.mask, P.mass32, P.res, P.tol_lo,
-                            P.tol_hi, 0.f, kout, j);
+        vk::k2_write(vk::k2_score<false>(fp, pt, frow[j], h_mfz[fhl[j]], P.seq_off, P.len, P.mask, P.mass32, P.res,
+                                         P.tol_lo, P.tol_hi, 0.f),
+                     vk::lnfact, kout, j);
     }
     __syncthreads();
     // ---------------------------------------------------------------- optional candidate outputs

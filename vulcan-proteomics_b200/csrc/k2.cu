@@ -3,17 +3,29 @@
 
 namespace {
 
-template <bool SHIFT>
+__global__ void __launch_bounds__(vk::KD_WARPS * 32, vk::KD_CTAS)
+k2_dense_k(vk_frag_params fpv, int n_spec, const int64_t* cand_off, const int32_t* c_row, const int8_t* c_maxfz,
+           const int64_t* pk_off, const float* pk_mass, const float* pk_int, const int64_t* seq_off,
+           const uint8_t* len, const uint64_t* mask, const float* mass32, const uint8_t* res, float tol_lo,
+           float tol_hi, vk::K2Out out) {
+  __shared__ vk::SmemFrag sf;
+  __shared__ vk::K2DenseSmem S;
+  vk::load_frag(sf, fpv);
+  __syncthreads();
+  vk::k2_dense_body(S, sf, n_spec, cand_off, c_row, c_maxfz, nullptr, pk_off, pk_mass, pk_int, seq_off, len, mask,
+                    mass32, res, tol_lo, tol_hi, out);
+}
+
 __global__ void __launch_bounds__(vk::K2_WARPS * 32)
-k2_spectra_k(vk_frag_params fpv, int n_spec, const int64_t* cand_off, const int32_t* c_row, const int8_t* c_maxfz,
-             const int64_t* pk_off, const float* pk_mass, const float* pk_int, const int64_t* seq_off,
-             const uint8_t* len, const uint64_t* mask, const float* mass32, const uint8_t* res, float tol_lo,
-             float tol_hi, const float* c_shift, vk::K2Out out) {
+k2_shift_k(vk_frag_params fpv, int n_spec, const int64_t* cand_off, const int32_t* c_row, const int8_t* c_maxfz,
+           const int64_t* pk_off, const float* pk_mass, const float* pk_int, const int64_t* seq_off,
+           const uint8_t* len, const uint64_t* mask, const float* mass32, const uint8_t* res, float tol_lo,
+           float tol_hi, const float* c_shift, vk::K2Out out) {
   __shared__ vk::SmemFrag sf;
   vk::load_frag(sf, fpv);
   __syncthreads();
-  vk::k2_body<SHIFT>(sf, n_spec, cand_off, c_row, c_maxfz, nullptr, pk_off, pk_mass, pk_int, seq_off, len, mask,
-                     mass32, res, tol_lo, tol_hi, c_shift, out);
+  vk::k2_body(sf, n_spec, cand_off, c_row, c_maxfz, nullptr, pk_off, pk_mass, pk_int, seq_off, len, mask, mass32, res,
+              tol_lo, tol_hi, c_shift, out);
 }
 
 // One thread per candidate (grid-stride over the run's candidates): the candidate's spectrum by binary search of
@@ -35,8 +47,9 @@ k2_cands_k(vk_frag_params fpv, int n_spec, const int64_t* cand_off, const int32_
     }
     const int64_t p0 = pk_off[lo];
     const vk::GlobalPeaks pt{pk_mass + p0, pk_int + p0, (int)min((int64_t)VK_K2_MAXPK, pk_off[lo + 1] - p0)};
-    vk::k2_score<false, vk::GlobalPeaks>(sf, pt, c_row[c], c_maxfz[c], seq_off, len, mask, mass32, res, tol_lo,
-                                         tol_hi, 0.f, out, c);
+    vk::k2_write(vk::k2_score<false, vk::GlobalPeaks>(sf, pt, c_row[c], c_maxfz[c], seq_off, len, mask, mass32, res,
+                                                      tol_lo, tol_hi, 0.f),
+                 vk::lnfact, out, c);
   }
 }
 
@@ -70,15 +83,17 @@ extern "C" int vk_k2_spectra(const vk_frag_params* fp, int n_spec, const int64_t
   if (!fp) return VK_E_ARG;
   if (n_spec <= 0) return 0;
   vk::K2Out out{o_hs, o_sb, o_sy, o_ppm, o_mb, o_my, o_lb, o_ly};
-  unsigned grid = (unsigned)((n_spec + vk::K2_WARPS - 1) / vk::K2_WARPS);
   cudaStream_t st = (cudaStream_t)stream;
-  if (c_shift)
-    k2_spectra_k<true><<<grid, vk::K2_WARPS * 32, 0, st>>>(*fp, n_spec, cand_off, c_row, c_maxfz, pk_off, pk_mass,
-                                                           pk_int, seq_off, len, mask, mass32, res, tol_lo, tol_hi,
-                                                           c_shift, out);
-  else
-    k2_spectra_k<false><<<grid, vk::K2_WARPS * 32, 0, st>>>(*fp, n_spec, cand_off, c_row, c_maxfz, pk_off, pk_mass,
-                                                            pk_int, seq_off, len, mask, mass32, res, tol_lo, tol_hi,
-                                                            nullptr, out);
+  if (c_shift) {
+    const unsigned grid = (unsigned)((n_spec + vk::K2_WARPS - 1) / vk::K2_WARPS);
+    k2_shift_k<<<grid, vk::K2_WARPS * 32, 0, st>>>(*fp, n_spec, cand_off, c_row, c_maxfz, pk_off, pk_mass, pk_int,
+                                                   seq_off, len, mask, mass32, res, tol_lo, tol_hi, c_shift, out);
+    return vk_launch_status();
+  }
+  int err = 0;
+  const int grid = vk::k2_dense_grid(k2_dense_k, n_spec, &err);
+  if (err) return err;
+  k2_dense_k<<<grid, vk::KD_WARPS * 32, 0, st>>>(*fp, n_spec, cand_off, c_row, c_maxfz, pk_off, pk_mass, pk_int,
+                                                 seq_off, len, mask, mass32, res, tol_lo, tol_hi, out);
   return vk_launch_status();
 }

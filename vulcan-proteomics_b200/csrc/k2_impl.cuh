@@ -1,11 +1,14 @@
 // K2 exact rescoring body (Sage score_candidate semantics, reference vulcan/gpu/kernels.cu:240-376).
 //
-// B200 launch shape: one warp per spectrum, K2_WARPS spectra per CTA.  The warp stages its spectrum's first 512
-// mass-sorted peaks in shared memory with a bucket table of start indices (one lookup + a short walk replaces the
-// reference's binary search; same index found); each lane scores whole candidates (the f32 sums are sequential in
-// ion order: b ions k ascending, fragment charge ascending, then y ions), so the per-candidate arithmetic is the
-// reference's operation for operation and the outputs are bit-identical.
+// Three launch shapes, with the same per-candidate arithmetic (the f32 sums are sequential in ion order: b ions k
+// ascending, fragment charge ascending, then y ions), which is the reference's operation for operation, so the
+// outputs are bit-identical: a CTA per spectrum for the closed scoring of dense lists (k2_dense_body), a warp per
+// spectrum for the shifted scoring (k2_body), a thread per candidate for sparse lists (k2_cands_k).  The first two
+// stage the spectrum's first 512 mass-sorted peaks in shared memory with a bucket table of start indices (one lookup
+// and a short walk replace the reference's binary search; same index found).
 #pragma once
+#include <math_constants.h>
+
 #include "common.cuh"
 
 namespace vk {
@@ -55,6 +58,11 @@ __device__ __forceinline__ int lower_bound_smem(const float* v, int n, float x) 
 // sm[j] < a: the same index the binary search returns, in one lookup and a short walk.
 constexpr int K2_BUCKETS = 512;
 
+__device__ __forceinline__ int k2_bucket(float x, float m0, float inv_w) {
+  const float t = __fmul_rn(__fsub_rn(x, m0), inv_w);
+  return t <= 0.f ? 0 : (t >= (float)(K2_BUCKETS - 1) ? K2_BUCKETS - 1 : (int)t);
+}
+
 struct PeakTable {
   const float* sm;
   const float* si;
@@ -62,11 +70,9 @@ struct PeakTable {
   int np;
   float m0, inv_w;
 
-  __device__ __forceinline__ int bucket(float x) const {
-    float t = __fmul_rn(__fsub_rn(x, m0), inv_w);
-    int b = t <= 0.f ? 0 : (t >= (float)(K2_BUCKETS - 1) ? K2_BUCKETS - 1 : (int)t);
-    return b;
-  }
+  __device__ __forceinline__ float mass(int j) const { return sm[j]; }
+  __device__ __forceinline__ float inten(int j) const { return si[j]; }
+  __device__ __forceinline__ int bucket(float x) const { return k2_bucket(x, m0, inv_w); }
   __device__ __forceinline__ int first_ge(float a) const {
     int j = start[bucket(a)];
     while (j < np && sm[j] < a) ++j;
@@ -102,6 +108,8 @@ struct GlobalPeaks {
   const float* si;
   int np;
 
+  __device__ __forceinline__ float mass(int j) const { return sm[j]; }
+  __device__ __forceinline__ float inten(int j) const { return si[j]; }
   __device__ __forceinline__ int first_ge(float a) const {
     int lo = 0, hi = np;
     while (lo < hi) {
@@ -112,13 +120,33 @@ struct GlobalPeaks {
   }
 };
 
+// A candidate's sums, counts and longest runs.
+struct K2Val {
+  float sb, sy, ppm;
+  int mb, my, lb, ly;
+};
+
+// Hyperscore and outputs of candidate c; lnf(n) is lnfact(n).
+template <class L>
+__device__ __forceinline__ void k2_write(const K2Val& v, L&& lnf, const K2Out& out, int64_t c) {
+  const double i2 = (double)__fadd_rn(v.sb, 1.0f) * (double)__fadd_rn(v.sy, 1.0f);
+  double hs = log(i2) + lnf(v.mb) + lnf(v.my);
+  if (!isfinite(hs)) hs = 255.0;
+  out.hs[c] = hs;
+  out.sb[c] = v.sb;
+  out.sy[c] = v.sy;
+  out.ppm[c] = __fdiv_rn(v.ppm, __fadd_rn(v.sb, v.sy));
+  out.mb[c] = (int16_t)v.mb;
+  out.my[c] = (int16_t)v.my;
+  out.lb[c] = (int16_t)v.lb;
+  out.ly[c] = (int16_t)v.ly;
+}
+
 template <bool SHIFT, class PT>
-__device__ __forceinline__ void k2_score(const SmemFrag& fp, const PT& pt, int r,
-                                         int maxfz, const int64_t* seq_off, const uint8_t* len,
-                                         const uint64_t* mask, const float* mass32, const uint8_t* res,
-                                         float tol_lo, float tol_hi, float shift, const K2Out& out, int64_t c) {
-  const float* sm = pt.sm;
-  const float* si = pt.si;
+__device__ __forceinline__ K2Val k2_score(const SmemFrag& fp, const PT& pt, int r,
+                                          int maxfz, const int64_t* seq_off, const uint8_t* len,
+                                          const uint64_t* mask, const float* mass32, const uint8_t* res,
+                                          float tol_lo, float tol_hi, float shift) {
   const int np = pt.np;
   const uint8_t* sq = res + seq_off[r];
   int L = len[r];
@@ -154,18 +182,18 @@ __device__ __forceinline__ void k2_score(const SmemFrag& fp, const PT& pt, int r
           float base = alt == 0 ? cum : __fadd_rn(cum, shift);
           float mz = z == 1 ? base : __fdiv_rn(base, (float)z);   // x / 1 == x exactly
           float a = tol_bound(mz, tol_lo, da), bd = tol_bound(mz, tol_hi, da);
-          for (int j = pt.first_ge(a); j < np && sm[j] <= bd; ++j) {
-            float it = si[j];
+          for (int j = pt.first_ge(a); j < np && pt.mass(j) <= bd; ++j) {
+            float it = pt.inten(j);
             if (it >= mx) { mx = it; best = j; best_mz = mz; }
             if (SHIFT && it >= mx_a) { mx_a = it; best_a = j; }
           }
           if (SHIFT && n_alt == 2 && best_a >= 0 && k < VK_K2_MAXLEN) {
-            if (alt == 0) { hit_u[kind][k] = __fadd_rn(hit_u[kind][k], si[best_a]); cnt_u[kind][k] += 1; }
-            else { hit_s[kind][k] = __fadd_rn(hit_s[kind][k], si[best_a]); cnt_s[kind][k] += 1; }
+            if (alt == 0) { hit_u[kind][k] = __fadd_rn(hit_u[kind][k], pt.inten(best_a)); cnt_u[kind][k] += 1; }
+            else { hit_s[kind][k] = __fadd_rn(hit_s[kind][k], pt.inten(best_a)); cnt_s[kind][k] += 1; }
           }
         }
         if (best >= 0) {
-          float pmass = sm[best], pint = si[best];
+          float pmass = pt.mass(best), pint = pt.inten(best);
           float num = __fmul_rn(__fmul_rn(pint, fabsf(__fsub_rn(best_mz, pmass))), 2.0e6f);
           ppm = __fadd_rn(ppm, __fdiv_rn(num, __fadd_rn(best_mz, pmass)));
           if (kind == 0) { mb += 1; sb = __fadd_rn(sb, pint); run_matched(rb, k); }
@@ -199,21 +227,422 @@ __device__ __forceinline__ void k2_score(const SmemFrag& fp, const PT& pt, int r
       if (h2 > best_hs) { best_hs = h2; mb = mb2; my = my2; sb = fmaxf(sb2, 0.f); sy = fmaxf(sy2, 0.f); }
     }
   }
-  double i2 = (double)__fadd_rn(sb, 1.0f) * (double)__fadd_rn(sy, 1.0f);
-  double hs = log(i2) + lnfact(mb) + lnfact(my);
-  if (!isfinite(hs)) hs = 255.0;
-  out.hs[c] = hs;
-  out.sb[c] = sb;
-  out.sy[c] = sy;
-  out.ppm[c] = __fdiv_rn(ppm, __fadd_rn(sb, sy));
-  out.mb[c] = (int16_t)mb;
-  out.my[c] = (int16_t)my;
-  out.lb[c] = (int16_t)rb.longest;
-  out.ly[c] = (int16_t)ry.longest;
+  return K2Val{sb, sy, ppm, mb, my, rb.longest, ry.longest};
 }
 
-// Warp-per-spectrum driver.  spec_ids == nullptr: spectrum bs uses peaks of spectrum bs.
-template <bool SHIFT>
+// ------------------------------------------------------------------------------------------ dense lists, closed
+//
+// One CTA of KD_WARPS warps per spectrum at a time, one lane per candidate.  Most
+// ions of a candidate meet no peak, and the lanes that do meet one differ from ion to ion, so a warp takes its
+// candidates in two loops instead of one lookup per ion:
+//   * walk (the ion index uniform over the warp): the running f32 masses of the b and y ions, each tested with one
+//     fused multiply-add and one bit of a presence bitmap (KD_BITS buckets of 1/KD_SCALE Th, wrapping around; a peak
+//     sets every bucket from which an ion could reach it, so a clear bit means no peak in the ion's window); the
+//     ions whose bit is set are marked in a mask and their masses listed in shared memory;
+//   * lookup: the listed ions of all the warp's candidates, 32 at a time with every lane busy: tolerance window, first
+//     peak by a table of start indices, most intense peak, its ppm term; then every lane adds its own ions' results,
+//     b then y in ion order.  The arithmetic is k2_score's, so the outputs are bit-identical to it.
+// Residues come four at a time from aligned words (single bytes where a word would leave the row), their masses
+// from one table of mono + delta, lnfact of small counts from a table built by the same function.  A
+// candidate of more than KD_MAXLEN residues, or with more marked ions than its lists hold, is scored by k2_score;
+// with fragment charges above 1 each lane looks its own ions up, charge by charge.
+//
+// What bounds it: instruction issue and the latency of a warp's dependent steps (the walk's shared-memory tests, the
+// lookup's search and division); HBM is at 5%.  The warp-per-spectrum kernel with a lookup per ion before it ran
+// 4,700 instructions per 32 candidates at 20.7 active lanes; this one runs 2,000 at 25.2.  Measured (device time per
+// launch, before -> now): 5.92M candidates of 40,000 spectra 1.590 -> 0.708 ms, 10,001 spectra of up to 1,000
+// candidates at 20 ppm 1.412 -> 0.37, fragment charges up to 3 1.078 -> 0.337, 32 spectra 0.030 -> 0.0105.
+// 3 warps per CTA at 8 CTAs per SM: 2, 4 and 6 warps took 12-16% longer on the 40,000 spectra (a spectrum's 148
+// candidates are 4.6 warps' worth; wider CTAs idle in their second round, narrower ones build the table with fewer).
+constexpr int KD_WARPS = 3;
+constexpr int KD_CTAS = 8;           // CTAs per SM (79 registers, 28 KB)
+constexpr int KD_LIST = 20;          // list slots per lane and kind (a group of four ions starts with four free)
+constexpr int KD_BITS = 8192;        // presence buckets
+constexpr float KD_SCALE = 4.0f;     // buckets per Th: 2,048 Th before they wrap
+constexpr int KD_LNF = 32;           // tabulated lnfact arguments
+constexpr int KD_MAXLEN = 65;        // residues whose 64 ions fit a mask
+constexpr int KD_QUEUE = 256;        // ions looked up per round of a warp (a lane has at most 2 * KD_LIST)
+static_assert(KD_QUEUE >= 2 * KD_LIST, "a lane's ions fit a round");
+
+struct K2DenseSmem {
+  float2 peak[VK_K2_MAXPK + 1];      // (mass, intensity), a NaN mass after the last
+  double lnf[KD_LNF];
+  uint32_t bits[KD_BITS / 32];
+  uint16_t start[K2_BUCKETS];        // first peak of 16 presence buckets (4 Th), from the first peak's on
+  float res[64];                     // residue mass by (letter & 31) | modified << 5
+  float ion[KD_WARPS][2][KD_LIST][32];   // listed ions' masses (b, y); after the lookup their peaks' intensities
+  float term[KD_WARPS][KD_QUEUE];        // ppm terms of the ions of a lookup round
+  uint16_t queue[KD_WARPS][KD_QUEUE];    // their places in ion
+};
+
+// Unwrapped bucket of mass m in the low bits: m * KD_SCALE rounded to an integer, monotone in m while its magnitude
+// stays below 2^21 (KD_SAFE); the low 13 bits are the bucket.
+constexpr float KD_SAFE = 2097152.0f / KD_SCALE;
+__device__ __forceinline__ uint32_t kd_bucket(float m) {
+  return __float_as_uint(__fmaf_rn(m, KD_SCALE, 12582912.0f));
+}
+__device__ __forceinline__ uint32_t kd_flag(const uint32_t* bits, float m) {
+  const uint32_t q = kd_bucket(m);
+  return __funnelshift_r(bits[(q >> 5) & (KD_BITS / 32 - 1)], 0u, q) & 1u;   // shift by q mod 32
+}
+
+// Ion masses that may have peak x in their tolerance window: [lo, hi] widened by 1e-6 of the masses, above the
+// rounding of the bounds, of this inversion and of the walk's approximate division by the charge.
+__device__ __forceinline__ float2 kd_reach(float x, float tol_lo, float tol_hi, int da) {
+  if (da) return make_float2((x - tol_hi) - 1e-6f * (fabsf(x) + fabsf(tol_hi)),
+                             (x - tol_lo) + 1e-6f * (fabsf(x) + fabsf(tol_lo)));
+  const float up = 1.f + tol_hi * 1e-6f, dn = 1.f + tol_lo * 1e-6f;
+  if (!(x > 0.f) || !(up > 0.5f && up < 2.f) || !(dn > 0.5f && dn < 2.f))
+    return make_float2(-CUDART_INF_F, CUDART_INF_F);
+  return make_float2(__fdividef(x, up) - 2e-6f * x, __fdividef(x, dn) + 2e-6f * x);
+}
+
+// Residues of a row, four per word, from aligned words of the table that hold no byte past the row (the first may
+// begin before it).
+struct RowWords {
+  const uint8_t* first;   // the table's first byte
+  const uint8_t* row;
+  const uint8_t* end;
+  const uint8_t* at;
+  uint32_t cur;
+
+  __device__ __forceinline__ uint32_t fetch(const uint8_t* a) const {
+    if (a >= first && a + 4 <= end) return __ldg(reinterpret_cast<const uint32_t*>(a));
+    uint32_t v = 0u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (a + j >= row && a + j < end) v |= (uint32_t)__ldg(a + j) << (8 * j);
+    return v;
+  }
+  __device__ __forceinline__ void begin(const uint8_t* table, const uint8_t* r, int len) {
+    first = table;
+    row = r;
+    end = r + len;
+    at = r - (reinterpret_cast<uintptr_t>(r) & 3);
+    cur = fetch(at);
+  }
+  __device__ __forceinline__ uint32_t next() {   // the next four residues (0 past the row)
+    at += 4;
+    const uint32_t nx = at < end ? fetch(at) : 0u;
+    const uint32_t r = __funnelshift_r(cur, nx, (uint32_t)(reinterpret_cast<uintptr_t>(row) & 3) * 8u);
+    cur = nx;
+    return r;
+  }
+};
+
+// Index of mass x into the start table whose first entry is bucket q0: monotone in x, clamped at both ends.
+__device__ __forceinline__ int kd_start(float x, uint32_t q0) {
+  const float t = fmaxf(__fmaf_rn(x, KD_SCALE, 12582912.0f), 8388608.0f);   // positive: its bits order like it
+  return min(max((int)(__float_as_uint(t) - q0), 0) >> 4, K2_BUCKETS - 1);
+}
+
+// The spectrum's table in the form k2_score takes.
+struct DensePeaks {
+  const K2DenseSmem& S;
+  int np;
+  uint32_t q0;
+  __device__ __forceinline__ float mass(int j) const { return S.peak[j].x; }
+  __device__ __forceinline__ float inten(int j) const { return S.peak[j].y; }
+  __device__ __forceinline__ int first_ge(float a) const {
+    int j = S.start[kd_start(a, q0)];
+    while (S.peak[j].x < a) ++j;   // ends at the NaN after the last peak
+    return j;
+  }
+};
+
+// The most intense peak (the last of equals) in the tolerance window of fragment m/z mz: its mass and intensity, a
+// NaN intensity when there is none.
+__device__ __forceinline__ float2 kd_match(const K2DenseSmem& S, uint32_t q0, float mz, float tol_lo, float tol_hi,
+                                           int da) {
+  const float a = tol_bound(mz, tol_lo, da), bd = tol_bound(mz, tol_hi, da);
+  const float2* pk = &S.peak[S.start[kd_start(a, q0)]];
+  float2 x = *pk;
+  while (x.x < a) x = *++pk;   // ends at the NaN after the last peak
+  float2 best = make_float2(0.f, CUDART_NAN_F);
+  while (x.x <= bd) {
+    if (x.y >= 0.f && !(x.y < best.y)) best = x;
+    x = *++pk;
+  }
+  return best;
+}
+
+__device__ __forceinline__ float kd_term(float mz, float2 peak) {
+  const float num = __fmul_rn(__fmul_rn(peak.y, fabsf(__fsub_rn(mz, peak.x))), 2.0e6f);
+  return __fdiv_rn(num, __fadd_rn(mz, peak.x));
+}
+
+static __device__ __noinline__ K2Val kd_score_serial(const SmemFrag* fp, const K2DenseSmem* S, int np, uint32_t q0,
+                                                     int r, int maxfz, const int64_t* seq_off,
+                                                     const uint8_t* len, const uint64_t* mask, const float* mass32,
+                                                     const uint8_t* res, float tol_lo, float tol_hi) {
+  const DensePeaks pt{*S, np, q0};
+  return k2_score<false, DensePeaks>(*fp, pt, r, maxfz, seq_off, len, mask, mass32, res, tol_lo, tol_hi, 0.f);
+}
+
+__device__ __forceinline__ double kd_lnfact(const K2DenseSmem& S, int n) {
+  return n < KD_LNF ? S.lnf[n] : lnfact(n);
+}
+
+// Longest run of consecutive matched ion indices (run_matched: ion 0 starts no run).
+__device__ __forceinline__ int kd_longest(uint64_t hit) {
+  int n = 0;
+  for (uint64_t x = hit & ~1ull; x; x &= x << 1) ++n;
+  return n;
+}
+
+// A candidate's row, loaded ahead of its scoring.
+struct DenseRow {
+  const uint8_t* seq;
+  uint64_t mask;
+  float mass;
+  int row, len, maxfz;
+
+  __device__ __forceinline__ int ions() const { return len <= KD_MAXLEN && maxfz > 1 ? len - 1 : 0; }
+};
+
+__device__ __forceinline__ DenseRow kd_row(int64_t c, const int32_t* c_row, const int8_t* c_maxfz,
+                                           const int64_t* seq_off, const uint8_t* len, const uint64_t* mask,
+                                           const float* mass32, const uint8_t* res) {
+  DenseRow d;
+  d.row = c_row[c];
+  d.maxfz = c_maxfz[c];
+  d.seq = res + seq_off[d.row];
+  d.len = len[d.row];
+  d.mask = mask[d.row];
+  d.mass = mass32[d.row];
+  return d;
+}
+
+// Scores the warp's candidates (lanes with `live` hold one each).
+__device__ __forceinline__ void kd_score(K2DenseSmem& S, const DensePeaks& pt, int warp, int lane, bool live,
+                                         const DenseRow& d, RowWords& w, const SmemFrag& fp, const int64_t* seq_off,
+                                         const uint8_t* len, const uint64_t* mask, const float* mass32,
+                                         const uint8_t* res, float tol_lo, float tol_hi, const K2Out& out,
+                                         int64_t c) {
+  const bool fits = live && d.len <= KD_MAXLEN;
+  const int n_ion = live ? d.ions() : 0;
+  const int n_max = __reduce_max_sync(VK_FULL, n_ion);
+  const int z_max = __reduce_max_sync(VK_FULL, fits ? d.maxfz : 0);
+  uint64_t mark_b = 0ull, mark_y = 0ull;   // ions that may match
+  bool over = false;
+  {
+    const float nt = nterm_of(fp, d.mask);
+    float b = nt, y = __fsub_rn(d.mass, nt);
+    int n_b = 0, n_y = 0;
+    for (int k0 = 0; k0 < n_max; k0 += 4) {
+      // a residue's table index per byte; past the row's end the index is 0, whose mass is 0: those ions land behind
+      // the list's valid part and their marks are cleared below
+      const bool in = k0 < n_ion;
+      uint32_t four = in ? w.next() & 0x1f1f1f1fu : 0u;
+      const uint32_t nib = (uint32_t)(d.mask >> k0) & 15u;
+      four |= ((nib * 0x00204081u) & 0x01010101u) << 5;
+      over |= in && max(n_b, n_y) > KD_LIST - 4;
+      float* list_b = &S.ion[warp][0][min(n_b, KD_LIST - 4)][lane];
+      float* list_y = &S.ion[warp][1][min(n_y, KD_LIST - 4)][lane];
+      uint32_t pb = 0u, py = 0u;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float rm = S.res[(four >> (8 * j)) & 63u];
+        b = __fadd_rn(b, rm);
+        y = __fsub_rn(y, rm);
+        uint32_t fb = kd_flag(S.bits, b), fy = kd_flag(S.bits, y);
+        for (int z = 2; z < z_max; ++z) {
+          const uint32_t on = z < d.maxfz;
+          fb |= on & kd_flag(S.bits, __fdividef(b, (float)z));
+          fy |= on & kd_flag(S.bits, __fdividef(y, (float)z));
+        }
+        if (in) {        // kept only when the slot moves on
+          *list_b = b;
+          *list_y = y;
+        }
+        list_b += fb * 32u;
+        list_y += fy * 32u;
+        pb += fb << j;
+        py += fy << j;
+      }
+      n_b += __popc(pb);
+      n_y += __popc(py);
+      mark_b |= (uint64_t)pb << k0;
+      mark_y |= (uint64_t)py << k0;
+    }
+  }
+  const uint64_t valid = n_ion < 64 ? (1ull << n_ion) - 1ull : ~0ull;
+  mark_b &= valid;
+  mark_y &= valid;
+  K2Val v{0.f, 0.f, 0.f, 0, 0, 0, 0};
+  uint64_t hit_b = 0ull, hit_y = 0ull;
+  if (z_max <= 2) {
+    const int n_b = __popcll(mark_b), n = over || !fits ? 0 : n_b + __popcll(mark_y);
+    const int end = (int)warp_incl_scan_i32(n), begin = end - n, total = __shfl_sync(VK_FULL, end, 31);
+    float* ion = &S.ion[warp][0][0][0];
+    for (int base = 0; base < total;) {   // the ions of as many whole lanes as a round holds: usually all
+      const bool mine = begin >= base && end <= base + KD_QUEUE && n > 0;
+      const int stop = __reduce_max_sync(VK_FULL, mine ? end : 0);
+      if (mine)
+        for (int i = 0; i < n; ++i)
+          S.queue[warp][begin - base + i] = (uint16_t)((i < n_b ? i : KD_LIST + i - n_b) * 32 + lane);
+      __syncwarp();
+      for (int t = lane; t < stop - base; t += 32) {
+        const int at = S.queue[warp][t];
+        const float mz = ion[at];
+        const float2 peak = kd_match(S, pt.q0, mz, tol_lo, tol_hi, fp.tol_da);
+        ion[at] = peak.y;
+        S.term[warp][t] = kd_term(mz, peak);
+      }
+      __syncwarp();
+      if (mine) {
+        const float* term = &S.term[warp][begin - base];
+        const float* at = &S.ion[warp][0][0][lane];
+        for (uint64_t todo = mark_b; todo; todo &= todo - 1ull, at += 32, ++term) {
+          const float pint = *at;
+          if (pint >= 0.f) {
+            v.ppm = __fadd_rn(v.ppm, *term);
+            v.mb += 1;
+            v.sb = __fadd_rn(v.sb, pint);
+            hit_b |= todo ^ (todo & (todo - 1ull));
+          }
+        }
+        at = &S.ion[warp][1][0][lane];
+        for (uint64_t todo = mark_y; todo; todo &= todo - 1ull, at += 32, ++term) {
+          const float pint = *at;
+          if (pint >= 0.f) {
+            v.ppm = __fadd_rn(v.ppm, *term);
+            v.my += 1;
+            v.sy = __fadd_rn(v.sy, pint);
+            hit_y |= todo ^ (todo & (todo - 1ull));
+          }
+        }
+      }
+      base = stop;
+      __syncwarp();
+    }
+  }
+  if (!live) return;
+  if (!fits || over) {
+    v = kd_score_serial(&fp, &S, pt.np, pt.q0, d.row, d.maxfz, seq_off, len, mask, mass32, res, tol_lo, tol_hi);
+  } else {
+    if (z_max > 2) {
+      uint64_t todo = mark_b;
+      bool in_y = todo == 0ull;
+      if (in_y) todo = mark_y;
+      const float* next = &S.ion[warp][in_y][0][lane];
+      while (todo) {   // the lane's marked ions, b then y
+        const uint64_t rest = todo & (todo - 1ull), bit = todo ^ rest;
+        todo = rest;
+        const float base = *next;
+        next += 32;
+        for (int z = 1; z < d.maxfz; ++z) {
+          const float mz = z == 1 ? base : __fdiv_rn(base, (float)z);   // x / 1 == x exactly
+          const float2 peak = kd_match(S, pt.q0, mz, tol_lo, tol_hi, fp.tol_da);
+          if (!(peak.y >= 0.f)) continue;
+          v.ppm = __fadd_rn(v.ppm, kd_term(mz, peak));
+          if (in_y) {
+            v.my += 1;
+            v.sy = __fadd_rn(v.sy, peak.y);
+            hit_y |= bit;
+          } else {
+            v.mb += 1;
+            v.sb = __fadd_rn(v.sb, peak.y);
+            hit_b |= bit;
+          }
+        }
+        if (!todo && !in_y) {
+          todo = mark_y;
+          in_y = true;
+          next = &S.ion[warp][1][0][lane];
+        }
+      }
+    }
+    v.lb = kd_longest(hit_b);
+    v.ly = kd_longest(hit_y);
+  }
+  k2_write(v, [&](int n) { return kd_lnfact(S, n); }, out, c);
+}
+
+// CTA-per-spectrum driver of the closed scoring.  spec_ids == nullptr: spectrum bs uses peaks of spectrum bs.
+__device__ __forceinline__ void k2_dense_body(K2DenseSmem& S, const SmemFrag& fp, int n_spec, const int64_t* cand_off,
+                                              const int32_t* c_row, const int8_t* c_maxfz, const int32_t* spec_ids,
+                                              const int64_t* pk_off, const float* pk_mass, const float* pk_int,
+                                              const int64_t* seq_off, const uint8_t* len, const uint64_t* mask,
+                                              const float* mass32, const uint8_t* res, float tol_lo, float tol_hi,
+                                              const K2Out& out) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int NT = KD_WARPS * 32;
+  const int da = fp.tol_da;
+  for (int i = tid; i < 64; i += NT) {
+    const int letter = (i & 31) - 1;
+    S.res[i] = letter >= 0 && letter < 26 ? __fadd_rn(fp.mono[letter], i & 32 ? fp.var[letter] : fp.stat[letter]) : 0.f;
+  }
+  if (warp == KD_WARPS - 1) S.lnf[lane] = lnfact(lane);
+  static_assert(KD_LNF == 32, "one entry per lane");
+  for (int bs = blockIdx.x; bs < n_spec; bs += gridDim.x) {
+    const int s = spec_ids ? spec_ids[bs] : bs;
+    const int64_t c0 = cand_off[bs], c1 = cand_off[bs + 1], p0 = pk_off[s], p1 = pk_off[s + 1];
+    if (c0 >= c1) continue;    // uniform over the CTA
+    const int np = (int)min((int64_t)VK_K2_MAXPK, p1 - p0);
+    DenseRow d{};              // this thread's first candidate, loaded while the table is built
+    const bool some = c0 + tid < c1;
+    if (some) d = kd_row(c0 + tid, c_row, c_maxfz, seq_off, len, mask, mass32, res);
+    __syncthreads();           // the previous spectrum's readers are done
+    for (int j = tid; j < np; j += NT) S.peak[j] = make_float2(pk_mass[p0 + j], pk_int[p0 + j]);
+    if (tid == 0) S.peak[max(np, 0)] = make_float2(CUDART_NAN_F, 0.f);
+    for (int j = tid; j < KD_BITS / 32; j += NT) S.bits[j] = 0u;
+    __syncthreads();
+    const float first = np > 0 ? S.peak[0].x : 0.f, last = np > 0 ? S.peak[np - 1].x : 0.f;
+    const DensePeaks pt{S, np, kd_bucket(first)};
+    for (int j = tid; j < np; j += NT) {
+      const float x = S.peak[j].x;
+      const float2 rg = kd_reach(x, tol_lo, tol_hi, da);
+      uint32_t qa = 0u, n = KD_BITS;   // the first bucket and how many
+      if (rg.x > -KD_SAFE && rg.y < KD_SAFE) {
+        qa = kd_bucket(rg.x);
+        n = min(kd_bucket(rg.y) - qa + 1u, (uint32_t)KD_BITS);
+      }
+      while (n > 0u) {
+        const uint32_t m = min(n, 32u - (qa & 31u));
+        atomicOr(&S.bits[(qa >> 5) & (KD_BITS / 32 - 1)], (0xffffffffu >> (32u - m)) << (qa & 31u));
+        qa += m;
+        n -= m;
+      }
+      const int b = kd_start(x, pt.q0);
+      const int bp = j > 0 ? kd_start(S.peak[j - 1].x, pt.q0) : -1;
+      for (int q = bp + 1; q <= b; ++q) S.start[q] = (uint16_t)j;
+    }
+    const int blast = np > 0 ? kd_start(last, pt.q0) : -1;
+    for (int q = blast + 1 + tid; q < K2_BUCKETS; q += NT) S.start[q] = (uint16_t)max(np, 0);
+    RowWords w;
+    w.cur = 0u;
+    if (some && d.ions() > 0) w.begin(res, d.seq, d.len);
+    __syncthreads();
+    for (int64_t cw = c0 + warp * 32; cw < c1; cw += NT) {   // uniform over the warp
+      const int64_t c = cw + lane;
+      kd_score(S, pt, warp, lane, c < c1, d, w, fp, seq_off, len, mask, mass32, res, tol_lo, tol_hi, out, c);
+      if (c + NT < c1) {
+        d = kd_row(c + NT, c_row, c_maxfz, seq_off, len, mask, mass32, res);
+        if (d.ions() > 0) w.begin(res, d.seq, d.len);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// Grid of a dense kernel: up to KD_WAVES CTAs per resident slot, each taking every grid-th spectrum -- enough CTAs
+// that the slots finish together (one per slot: 62 us instead of 44 on 5,000 spectra, 428 instead of 370 on 10,001),
+// few enough that a CTA's residue and lnfact tables serve several spectra.
+constexpr int KD_WAVES = 8;
+template <class F>
+int k2_dense_grid(F kernel, int n_spec, int* err) {
+  int per_sm = 0, dev = 0, n_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, KD_WARPS * 32, 0);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  *err = (int)e;
+  if (e != cudaSuccess) return 0;
+  const int most = (per_sm > 1 ? per_sm : 1) * n_sm * KD_WAVES;
+  return most < n_spec ? most : n_spec;
+}
+
+// Warp-per-spectrum driver of the shifted scoring.  spec_ids == nullptr: spectrum bs uses peaks of spectrum bs.
 __device__ __forceinline__ void k2_body(const SmemFrag& fp, int n_spec, const int64_t* cand_off,
                                         const int32_t* c_row, const int8_t* c_maxfz, const int32_t* spec_ids,
                                         const int64_t* pk_off, const float* pk_mass, const float* pk_int,
@@ -239,9 +668,9 @@ __device__ __forceinline__ void k2_body(const SmemFrag& fp, int n_spec, const in
     const PeakTable pt = build_table(sm, si, s_start[warp], np, lane);
     int64_t c1 = cand_off[bs + 1];
     for (int64_t c = cand_off[bs] + lane; c < c1; c += 32) {
-      float shift = SHIFT ? c_shift[c] : 0.f;
-      k2_score<SHIFT, PeakTable>(fp, pt, c_row[c], c_maxfz[c], seq_off, len, mask, mass32, res, tol_lo, tol_hi,
-                                 shift, out, c);
+      k2_write(k2_score<true, PeakTable>(fp, pt, c_row[c], c_maxfz[c], seq_off, len, mask, mass32, res, tol_lo, tol_hi,
+                                         c_shift[c]),
+               lnfact, out, c);
     }
   }
 }
