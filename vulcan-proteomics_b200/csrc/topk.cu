@@ -2,9 +2,11 @@
 //
 // The reference sorts every appended (hyp, row, count) of the run by a packed key
 // (spectrum, 32767 - min(count, 32767), 2^28 - 1 - row) and keeps rank < topk per spectrum, then adds partner rows
-// and merges duplicates of (spectrum, row) to the lowest hypothesis and highest count.  Here a warp reads its
-// spectrum's dense K1 counts once (loads unrolled), computing the per-hypothesis scored/matched statistics and
-// collecting the appended entries as unique 63-bit keys (min(count,32767), row, -hypothesis) in shared memory;
+// and merges duplicates of (spectrum, row) to the lowest hypothesis and highest count.  Spectra whose windows are
+// disjoint -- nearly all -- take select_topk_rows_k, which needs no sort (below).  The others take select_topk_k: a
+// warp reads its spectrum's dense K1 counts once (loads unrolled), computing the per-hypothesis scored/matched
+// statistics and collecting the appended entries as unique 63-bit keys (min(count,32767), row, -hypothesis) in shared
+// memory;
 //   - if at most topk entries pass the threshold, takes them all;
 //   - otherwise finds the topk-th largest key by an 8-bit radix select over the collected keys and keeps the keys
 //     at or above it (keys are unique, so exactly topk);
@@ -128,15 +130,244 @@ __device__ __forceinline__ int64_t win_rows(int64_t w0, int64_t lo, int64_t hi, 
   return w0 + n <= cnt_cap ? n : 0;
 }
 
+// ------------------------------------------------------------------------------------------ disjoint windows
+//
+// Every window row is one hypothesis' alone, so (visiting the windows in row order) a bit per window row says all:
+//   1. the counts are read once into a histogram, which gives the count T of the topk-th entry and how many entries
+//      tie at T;
+//   2. a second read (L1 / L2) marks the rows above T, and the last of the tied ones (ties go to the higher row);
+//   3. the partner of every marked row is marked in a second bitmap;
+//   4. the rows of the union come out in order: position by prefix popcounts, count from the marked rows' list.
+// 4.2k warp instructions per spectrum of 850 window rows at topk 100, where collecting keys, radix-selecting and
+// sorting them took 10.8k; bound by issue (0.67 a cycle) and the L2 latency of the counts.  Measured per launch,
+// before -> now: 40,000 spectra at topk 100 0.725 -> 0.203 ms, 16,384 with 2,100 window rows each at topk 200
+// 1.588 -> 0.178, 10,001 at topk 500 1.112 -> 0.113, 32 spectra 0.009 -> 0.0064 (and 0.002 for the launch that looks
+// for what was left over).  Staging the rows of step 4 in shared memory for whole-sector writes was slower (0.228 and
+// 0.142: fewer warps per SM), and so was a tally in byte fields of registers (0.216).  What does not fit goes to select_topk_k by n_cand = -1: more than 32
+// hypotheses or overlapping windows, more than TR_WORDS * 32 window rows, a count above 254, a partner outside its
+// own hypothesis' window.
+constexpr int TR_WORDS = 384;        // bitmap words per spectrum: 12,288 window rows
+constexpr int TR_TOPK = 512;         // longest list
+
+struct __align__(16) RowsScratch {   // per warp, the windows in row order
+  int64_t lo[32], w0[32];
+  int32_t n[32], hl[32], word[32];
+  uint32_t mark[TR_WORDS], all[TR_WORDS];
+};
+
 __global__ void __launch_bounds__(TK_WARPS * 32)
-select_topk_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi, const int64_t* win_off,
+select_topk_rows_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
+                   const int64_t* win_off, const int32_t* __restrict__ cnt, int64_t cnt_cap, const int64_t* partner,
+                   int thr, int topk, int pair_closure, int cap, int list_len, int64_t* c_hyp, int64_t* c_row,
+                   int64_t* c_cnt, int64_t* n_cand, uint32_t* hyp_scored, uint64_t* hyp_matched,
+                   int64_t* spec_scored, int64_t* spec_matched) {
+  extern __shared__ __align__(16) uint8_t tk_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s = blockIdx.x * TK_WARPS + warp;
+  if (s >= n_spec) return;
+  uint8_t* base = tk_smem + (sizeof(RowsScratch) + (size_t)list_len * 4) * warp;
+  RowsScratch& W = *reinterpret_cast<RowsScratch*>(base);
+  // the histogram of the counts (step 1), then the marked rows in order: bitmap place << 13 | window << 8 | count
+  uint32_t* list = reinterpret_cast<uint32_t*>(base + sizeof(RowsScratch));
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const int64_t hb = spec_hyp_off[s];
+  const int nhs = (int)min(spec_hyp_off[s + 1] - hb, (int64_t)33);
+  bool fit = nhs <= 32;
+  int words = 0;
+  if (fit) {   // lane h: window of hypothesis hb + h; its rank in row order (empty windows last), its first word
+    const bool mine = lane < nhs;
+    const int64_t lo = mine ? h_lo[hb + lane] : 0, w0 = mine ? win_off[hb + lane] : 0;
+    const int64_t n = mine ? win_rows(w0, lo, h_hi[hb + lane], cnt_cap) : 0, hi = lo + n;
+    int rank = 0;
+    bool bad = n > TR_WORDS * 32;
+    for (int j = 0; j < nhs; ++j) {
+      const int64_t lo_j = __shfl_sync(VK_FULL, lo, j), hi_j = __shfl_sync(VK_FULL, hi, j);
+      const bool live_j = hi_j > lo_j;
+      if (n > 0) {
+        rank += live_j && (lo_j < lo || (lo_j == lo && j < lane));
+        bad |= live_j && j != lane && lo_j < hi && lo < hi_j;
+      } else {
+        rank += live_j || j < lane;
+      }
+    }
+    fit = !__any_sync(VK_FULL, bad);
+    if (fit && mine) {
+      W.lo[rank] = lo;
+      W.w0[rank] = w0;
+      W.n[rank] = (int32_t)n;
+      W.hl[rank] = lane;
+    }
+    __syncwarp();
+    const int nw = fit && mine ? (W.n[lane] + 31) >> 5 : 0;
+    const int end = vk::warp_incl_scan_i32(nw);
+    if (mine) W.word[lane] = end - nw;
+    words = __shfl_sync(VK_FULL, end, 31);
+    fit = fit && words <= TR_WORDS;
+  }
+  if (!fit) {
+    if (lane == 0) n_cand[s] = -1;
+    return;
+  }
+  for (int i = lane; i < 256; i += 32) list[i] = 0u;
+  __syncwarp();
+  // 1. statistics and the histogram of the counts (increments by one of the same word are aggregated in hardware)
+  long long s_sc = 0, s_mt = 0;
+  for (int r = 0; r < nhs; ++r) {
+    const int n = W.n[r];
+    const int32_t* src = cnt + W.w0[r];
+    uint32_t sc = 0u, mt = 0u;
+    for (int j0 = 0; j0 < n; j0 += 32 * TK_UNROLL) {
+      int c[TK_UNROLL];
+#pragma unroll
+      for (int u = 0; u < TK_UNROLL; ++u) {
+        const int j = j0 + 32 * u + lane;
+        c[u] = j < n ? src[j] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < TK_UNROLL; ++u) {
+        mt += (uint32_t)c[u];
+        if (c[u] > 0) {
+          ++sc;
+          atomicAdd(&list[min(c[u], 255)], 1u);
+        }
+      }
+    }
+    const long long sc_w = __reduce_add_sync(VK_FULL, sc), mt_w = vk::warp_sum((long long)mt);
+    if (lane == 0) {
+      hyp_scored[hb + W.hl[r]] = (uint32_t)sc_w;
+      hyp_matched[hb + W.hl[r]] = (uint64_t)mt_w;
+    }
+    s_sc += sc_w;
+    s_mt += mt_w;
+  }
+  if (lane == 0 && spec_scored) {
+    spec_scored[s] = s_sc;
+    spec_matched[s] = s_mt;
+  }
+  __syncwarp();
+  // T: every entry above it is taken, and of the entries at it all but the first `skip`.  Lane l holds the counts
+  // 8 l .. 8 l + 7 that are entries; the topk-th is in the highest lane with more than topk entries at or above it
+  int T = thr - 1, skip = 0;
+  {
+    uint32_t mine = 0u;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) mine += 8 * lane + q >= thr ? list[8 * lane + q] : 0u;
+    uint32_t suffix = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_down_sync(VK_FULL, suffix, o);
+      if (lane + o < 32) suffix += v;
+    }
+    const unsigned hold = __ballot_sync(VK_FULL, suffix > (uint32_t)topk);
+    if (hold) {
+      const int l = 31 - __clz(hold);
+      uint32_t above = __shfl_sync(VK_FULL, suffix - mine, l);
+      for (int q = 7; q >= 0; --q) {
+        const uint32_t v = list[8 * l + q];
+        if (above + v > (uint32_t)topk) {
+          T = 8 * l + q;
+          skip = (int)(above + v) - topk;
+          break;
+        }
+        above += v;
+      }
+    }
+  }
+  if (list[255]) {   // (uniform) a count above 254
+    if (lane == 0) n_cand[s] = -1;
+    return;
+  }
+  __syncwarp();
+  // 2. mark the taken rows
+  const bool tied = skip > 0;
+  int n_sel = 0, seen = 0;
+  for (int r = 0; r < nhs; ++r) {
+    const int n = W.n[r], w_r = W.word[r];
+    const int32_t* src = cnt + W.w0[r];
+    for (int j0 = 0; j0 < n; j0 += 128) {
+      int c[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = j0 + 32 * u + lane;
+        c[u] = j < n ? src[j] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (j0 + 32 * u >= n) break;   // uniform
+        unsigned take = __ballot_sync(VK_FULL, c[u] > T);
+        if (tied) {
+          unsigned eq = __ballot_sync(VK_FULL, c[u] == T);
+          const int k = __popc(eq);
+          for (int i = seen; i < skip && eq; ++i) eq &= eq - 1u;   // the first `skip` tied rows are left out
+          seen += k;
+          take |= eq;
+        }
+        const int w = w_r + ((j0 + 32 * u) >> 5);
+        if (lane == 0) {
+          W.mark[w] = take;
+          W.all[w] = take;
+        }
+        if ((take >> lane) & 1u)
+          list[n_sel + __popc(take & lt_mask)] =
+              ((uint32_t)(w * 32 + lane) << 13) | ((uint32_t)r << 8) | (uint32_t)c[u];
+        n_sel += __popc(take);
+      }
+    }
+  }
+  __syncwarp();
+  // 3. partners
+  if (pair_closure) {
+    bool out = false;
+    for (int i = lane; i < n_sel; i += 32) {
+      const uint32_t e = list[i];
+      const int r = (int)(e >> 8) & 31, at = (int)(e >> 13) - 32 * W.word[r];
+      const int64_t p = partner[W.lo[r] + at] - W.lo[r];
+      if (p >= 0 && p < W.n[r]) atomicOr(&W.all[W.word[r] + (int)(p >> 5)], 1u << (p & 31));
+      else out = true;
+    }
+    if (__any_sync(VK_FULL, out)) {
+      if (lane == 0) n_cand[s] = -1;
+      return;
+    }
+  }
+  __syncwarp();
+  // 4. the rows of the union, a word per lane
+  int carry = 0;   // rows and marked rows before this chunk of words: low and high half
+  const int64_t slot = (int64_t)s * cap;
+  for (int w0 = 0; w0 < words; w0 += 32) {
+    const int w = w0 + lane;
+    uint32_t u = w < words ? W.all[w] : 0u;
+    const uint32_t m = w < words ? W.mark[w] : 0u;
+    const int both = __popc(u) | (__popc(m) << 16);
+    const int end = vk::warp_incl_scan_i32(both) + carry;
+    int at = (end - both) & 0xffff, li = (end - both) >> 16;
+    int r = 0;
+    while (r + 1 < nhs && W.word[r + 1] <= w && W.n[r + 1] > 0) ++r;
+    const int64_t h = hb + W.hl[r], row0 = W.lo[r] + 32 * (w - W.word[r]);
+    while (u) {
+      const int b = __ffs(u) - 1;
+      u &= u - 1u;
+      int c = -1;
+      if ((m >> b) & 1u) c = (int)(list[li++] & 255u);
+      c_hyp[slot + at] = h;
+      c_row[slot + at] = row0 + b;
+      c_cnt[slot + at] = c;
+      ++at;
+    }
+    carry = __shfl_sync(VK_FULL, end, 31);
+  }
+  if (lane == 0) n_cand[s] = carry & 0xffff;
+}
+
+// ------------------------------------------------------------------------------------------ any windows
+// One spectrum per warp; rest: only the spectra select_topk_rows_k left (n_cand = -1).
+__global__ void __launch_bounds__(TK_WARPS * 32)
+select_topk_k(int n_spec, int rest, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi, const int64_t* win_off,
               const int32_t* cnt, int64_t cnt_cap, const int64_t* partner, int thr, int topk, int pair_closure, int cap,
               int list_pow2, int key_cap, int64_t* c_hyp, int64_t* c_row, int64_t* c_cnt, int64_t* n_cand,
               uint32_t* hyp_scored, uint64_t* hyp_matched, int64_t* spec_scored, int64_t* spec_matched) {
   extern __shared__ __align__(16) uint8_t tk_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int s = blockIdx.x * TK_WARPS + warp;
-  if (s >= n_spec) return;
   const size_t per_warp = (size_t)key_cap * 8 + (size_t)list_pow2 * (4 + 4 + 4) + 256 * 4;
   uint8_t* base = tk_smem + per_warp * warp;
   WarpLists W;
@@ -147,6 +378,7 @@ select_topk_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, cons
   W.hist = reinterpret_cast<uint32_t*>(W.cnt + list_pow2);
   const unsigned lt_mask = (1u << lane) - 1u;
 
+  auto one = [&](int s) {
   const int64_t hb = spec_hyp_off[s], he = spec_hyp_off[s + 1];
   // one read of the counts: per-hypothesis statistics, and the appended keys into shared memory (as many as fit)
   long long n_app = 0, s_sc = 0, s_mt = 0;
@@ -295,6 +527,17 @@ select_topk_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, cons
     n_out += __popc(m);
   }
   if (lane == 0) n_cand[s] = n_out;
+  __syncwarp();
+  };
+  const int step = gridDim.x * TK_WARPS, first = blockIdx.x * TK_WARPS + warp;
+  if (!rest) {
+    for (int s = first; s < n_spec; s += step) one(s);
+    return;
+  }
+  for (int s0 = first * 32; s0 < n_spec; s0 += step * 32) {
+    unsigned left = __ballot_sync(VK_FULL, s0 + lane < n_spec && n_cand[s0 + lane] < 0);
+    for (; left; left &= left - 1u) one(s0 + __ffs(left) - 1);
+  }
 }
 
 // Per-warp scratch of the hit reader: up to 32 hypotheses in visiting order and one chunk of 32 segments.
@@ -797,6 +1040,9 @@ compact_k(int n_spec, int cap, const int64_t* n_cand, const int64_t* cand_off, c
   }
 }
 
+// Whether select_topk_rows_k takes the call (rows with a zero count are entries only for the general kernel).
+int topk_by_rows(int thr, int topk) { return thr >= 1 && thr <= 254 && topk <= TR_TOPK; }
+
 }  // namespace
 
 extern "C" {
@@ -817,11 +1063,26 @@ int vk_select_topk(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   if (sh > 220 * 1024) return VK_E_ARG;
   cudaError_t e = cudaFuncSetAttribute(select_topk_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (e != cudaSuccess) return vk_err(e);
-  select_topk_k<<<(unsigned)((n_spec + TK_WARPS - 1) / TK_WARPS), TK_WARPS * 32, sh, (cudaStream_t)stream>>>(
-      n_spec, spec_hyp_off, h_lo, h_hi, win_off, cnt, cnt_cap, partner, thr, topk, pair_closure, cap, list_pow2,
-      key_cap, c_hyp,
-      c_row,
-      c_cnt, n_cand, hyp_scored, hyp_matched, spec_scored, spec_matched);
+  const unsigned blocks = (unsigned)((n_spec + TK_WARPS - 1) / TK_WARPS);
+  unsigned grid = blocks;
+  const int rest = topk_by_rows(thr, topk);
+  if (rest) {
+    const int list_len = ((topk > 256 ? topk : 256) + 3) & ~3;   // each warp's scratch on a 16-byte boundary
+    const size_t rsh = (sizeof(RowsScratch) + (size_t)list_len * 4) * TK_WARPS;
+    e = cudaFuncSetAttribute(select_topk_rows_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsh);
+    if (e != cudaSuccess) return vk_err(e);
+    select_topk_rows_k<<<blocks, TK_WARPS * 32, rsh, (cudaStream_t)stream>>>(
+        n_spec, spec_hyp_off, h_lo, h_hi, win_off, cnt, cnt_cap, partner, thr, topk, pair_closure, cap, list_len,
+        c_hyp, c_row, c_cnt, n_cand, hyp_scored, hyp_matched, spec_scored, spec_matched);
+    const int rc = vk_launch_status();
+    if (rc != 0) return rc;
+    // a few CTAs look for the spectra left over, 32 flags at a time
+    grid = (unsigned)((n_spec + TK_WARPS * 32 - 1) / (TK_WARPS * 32));
+    if (grid > 296u) grid = 296u;
+  }
+  select_topk_k<<<grid, TK_WARPS * 32, sh, (cudaStream_t)stream>>>(
+      n_spec, rest, spec_hyp_off, h_lo, h_hi, win_off, cnt, cnt_cap, partner, thr, topk, pair_closure, cap, list_pow2,
+      key_cap, c_hyp, c_row, c_cnt, n_cand, hyp_scored, hyp_matched, spec_scored, spec_matched);
   return vk_launch_status();
 }
 

@@ -950,6 +950,7 @@ def _shortlist(gi: GpuIndex, p: SearchParams, n: int, dh, win_off, cnt, topk: in
     dev = gi.dev
     n_h = dh["n_max"]
     cap = (2 if closure else 1) * topk
+    thr = p.k1_threshold if thr is None else thr
     s_hyp = torch.empty(max(n * cap, 1), dtype=torch.int64, device=dev)
     s_row = torch.empty_like(s_hyp)
     s_cnt = torch.empty_like(s_hyp)
@@ -959,11 +960,11 @@ def _shortlist(gi: GpuIndex, p: SearchParams, n: int, dh, win_off, cnt, topk: in
     spec_scored = torch.empty(max(n, 1), dtype=torch.int64, device=dev)
     spec_matched = torch.empty(max(n, 1), dtype=torch.int64, device=dev)
     K.check(L.vk_select_topk(n, K.ptr(dh["spec_off"]), K.ptr(dh["lo"]), K.ptr(dh["hi"]), K.ptr(win_off),
-                             K.ptr(cnt), cnt.numel(), K.ptr(gi.partner), p.k1_threshold if thr is None else thr, topk,
+                             K.ptr(cnt), cnt.numel(), K.ptr(gi.partner), thr, topk,
                              int(closure), cap,
                              K.ptr(s_hyp), K.ptr(s_row), K.ptr(s_cnt), K.ptr(n_cand), K.ptr(hyp_scored),
                              K.ptr(hyp_matched), K.ptr(spec_scored), K.ptr(spec_matched), K.stream()),
-            "select_topk")
+            "select_topk", 2 if 1 <= thr <= 254 and topk <= 512 else 1)
     cand = _compact(n, cap, n_cand, s_hyp, s_row, s_cnt, dh, dev)
     sums = {"hyp_scored": hyp_scored, "hyp_matched": hyp_matched, "spec_scored": spec_scored,
             "spec_matched": spec_matched}
