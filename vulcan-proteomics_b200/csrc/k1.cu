@@ -110,9 +110,19 @@ __device__ __forceinline__ K1Rec k1_record(int64_t it, int64_t r0, int T, const 
 // item's chain of dependent loads (item -> hypothesis -> spectrum) overlaps the copy and the other items'.  Warp w
 // then runs the filtered per-item search of items w, w + warps, ... (measured faster than items taken one at a time
 // through a shared-memory counter).
-// HITS: the hit-list form (K1Hits) instead of the dense counts.
-template <bool HITS>
-__global__ void __launch_bounds__(K1_MAX_WARPS * 32, 1)
+// HITS: the hit-list form (K1Hits) instead of the dense counts.  ISUM: with intensity sums.
+//
+// What bounds it: reading the tiles takes 0.45 of the time at 20,000 spectra on 5.7M rows (0.176 of 0.386 ms with no
+// item worked on: 0.98 GB, at 85% of the copy rate); the rest is issue and the latency of each warp's steps (0.45
+// instructions a cycle, 8 CTAs per SM), of which the exact searches take 0.13 ms, the filter 0.055, clearing and
+// writing the histograms 0.03.  Against the form before -- filter words loaded when needed, a second path for windows
+// that straddle a bitmap word, a search per coarse bin, run-time intensity branches -- a launch took, before -> now:
+// dense, 40,000 spectra 0.725 -> 0.570 ms; hit lists with intensity sums 0.801 -> 0.703; fragment charges up to 3
+// 0.637 -> 0.487; open windows 0.316 -> 0.236.  Not kept: starting a window's scan at the popcount of the bitmap bits
+// below it instead of a binary search (0.71: isobaric fragments crowd single bits, so the scans are long); one word a
+// lane ahead 0.64, three 0.58; without a register limit the compiler takes 75-80 and one or two CTAs fewer fit.
+template <bool HITS, bool ISUM>
+__global__ void __maxnreg__((ISUM ? 80 : 72))
 k1_tiles_k(vk_tindex ix, float tol_lo, float tol_hi, int tol_da, int post_cap, const int64_t* tile_item_off,
            const int32_t* item_hyp, int64_t n_hyp, int64_t item_cap, const int32_t* h_spec, const int8_t* h_maxfz,
            const int64_t* h_lo, const int64_t* h_hi, const int64_t* win_off, int64_t cnt_cap, const int64_t* pk_off,
@@ -150,15 +160,20 @@ k1_tiles_k(vk_tindex ix, float tol_lo, float tol_hi, int tol_da, int post_cap, c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t* qw = queue + warp * vk::K1_QUEUE;
   uint32_t* hw = hist + warp * T;
-  uint32_t* iw = isum_out ? ihist + warp * T : nullptr;
+  uint32_t* iw = ihist + warp * T;   // (ISUM)
+  const uint32_t bm_mask = (uint32_t)(nb * vk::K1_BM_WORDS - 1);
   const int64_t r0 = t << ix.tile_shift;
   bool staged = false;
   for (int64_t c0 = i0; c0 < i1; c0 += K1_ITEMS) {
     const int m = (int)min((int64_t)K1_ITEMS, i1 - c0);
     for (int j = threadIdx.x; j < m; j += blockDim.x)
       rec[j] = k1_record(c0 + j, r0, T, item_hyp, n_hyp, h_spec, h_maxfz, h_lo, h_hi, win_off, cnt_cap, pk_off,
-                         tic, iw != nullptr, status);
+                         tic, ISUM, status);
     __syncthreads();
+    // the words of the warp's first item (before the wait for the tile); each item then loads the next one's
+    vk::K1Words words;
+    auto peaks_of = [&](int j) { return j < m && rec[j].mfz > 1 ? rec[j].n : 0; };
+    if (n_kz > 0) words.load(pk_filt + (peaks_of(warp) ? rec[warp].p0 : 0) + lane, peaks_of(warp), 0, lane);
     if (!staged) {
       // CTA-uniform decision: later rounds begin with CTA barriers
       if (!__syncthreads_and(vk::mbar_wait(&bar, 0, WAIT_LIMIT))) {
@@ -171,16 +186,21 @@ k1_tiles_k(vk_tindex ix, float tol_lo, float tol_hi, int tol_da, int post_cap, c
     }
     for (int j = warp; j < m; j += n_warps) {
       const K1Rec r = rec[j];
-      if (r.mfz == 0) continue;
+      const int next_n = peaks_of(j + n_warps);
+      const int64_t next_p0 = next_n ? rec[j + n_warps].p0 : 0;
+      if (r.mfz == 0) {
+        if (n_kz > 0) words.load(pk_filt + next_p0 + lane, next_n, 0, lane);
+        continue;
+      }
       const int rlo = r.rows & 0xffff, rhi = r.rows >> 16;
-      for (int q = rlo + lane; q < rhi; q += 32) {
-        hw[q] = 0;
-        if (iw) iw[q] = 0;
+      for (int q = lane * 4; q < T; q += 128) {
+        *reinterpret_cast<uint4*>(hw + q) = make_uint4(0u, 0u, 0u, 0u);
+        if (ISUM) *reinterpret_cast<uint4*>(iw + q) = make_uint4(0u, 0u, 0u, 0u);
       }
       __syncwarp();
-      vk::k1_item_filtered(post, cb, bm, hw, iw, rlo, rhi, r.p0, r.p0 + r.n,
-                           r.mfz, pk_keys, pk_filt, n_kz, kstride, pk_mass, tol_lo, tol_hi, tol_da, ix, lane, qw,
-                           pk_int, r.ws);
+      vk::k1_item_filtered<ISUM>(post, cb, bm, bm_mask, hw, iw, rlo, rhi, r.p0, r.n, r.mfz, pk_keys, pk_filt, n_kz,
+                                 kstride, pk_mass, tol_lo, tol_hi, tol_da, ix, lane, qw, pk_int, r.ws, words, next_p0,
+                                 next_n);
       __syncwarp();
       if (HITS) {
         // the item's segment: the slots of the window rows rlo..rhi of this tile (r.base is the region index of
@@ -200,7 +220,7 @@ k1_tiles_k(vk_tindex ix, float tol_lo, float tol_hi, int tol_da, int post_cap, c
           if (keep) {
             const int64_t at = seg + n_kept + __popc(bal & ((1u << lane) - 1u));
             hits.rc[at] = ((uint64_t)c << 32) | (uint64_t)(r0 + q);
-            if (iw) hits.isum[at] = iw[q];
+            if (ISUM) hits.isum[at] = iw[q];
           }
           n_kept += __popc(bal);
         }
@@ -215,7 +235,7 @@ k1_tiles_k(vk_tindex ix, float tol_lo, float tol_hi, int tol_da, int post_cap, c
       } else {
         for (int q = rlo + lane; q < rhi; q += 32) {
           cnt[r.base + q] = (int32_t)hw[q];
-          if (iw) isum_out[r.base + q] = iw[q];
+          if (ISUM) isum_out[r.base + q] = iw[q];
         }
       }
       __syncwarp();
@@ -277,7 +297,7 @@ int vk_k1_plan_fill(const vk_tindex* ix, int64_t n_hyp, const int64_t* h_lo, con
 
 namespace {
 
-template <bool HITS>
+template <bool HITS, bool ISUM>
 int k1_tiles_launch(const vk_tindex* ix, const vk_frag_params* fp, float tol_lo, float tol_hi, int warps,
                     const int64_t* tile_item_off, const int32_t* item_hyp, int64_t n_hyp, int64_t item_cap,
                     const int32_t* h_spec, const int8_t* h_maxfz, const int64_t* h_lo, const int64_t* h_hi,
@@ -293,13 +313,13 @@ int k1_tiles_launch(const vk_tindex* ix, const vk_frag_params* fp, float tol_lo,
   const int T = 1 << ix->tile_shift;
   const int nb = 1 << ix->cbin_bits;
   const int stride = (nb + 1 + 7) & ~7;
-  if (isum && (!pk_int || !tic)) return VK_E_ARG;
+  if (ISUM && (!pk_int || !tic)) return VK_E_ARG;
   const size_t sh = (size_t)ix->max_tile_postings * 4 + (size_t)stride * 2 + (size_t)nb * vk::K1_BM_WORDS * 4 +
-                    (size_t)warps * (T * 4 * (isum ? 2 : 1) + vk::K1_QUEUE * 4);
+                    (size_t)warps * (T * 4 * (ISUM ? 2 : 1) + vk::K1_QUEUE * 4);
   if (sh > 200 * 1024) return VK_E_TOO_LARGE;
-  cudaError_t e = cudaFuncSetAttribute(k1_tiles_k<HITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  cudaError_t e = cudaFuncSetAttribute(k1_tiles_k<HITS, ISUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (e != cudaSuccess) return vk_err(e);
-  k1_tiles_k<HITS><<<(unsigned)ix->n_tiles, warps * 32, sh, (cudaStream_t)stream>>>(
+  k1_tiles_k<HITS, ISUM><<<(unsigned)ix->n_tiles, warps * 32, sh, (cudaStream_t)stream>>>(
       *ix, tol_lo, tol_hi, fp->tol_da, ix->max_tile_postings, tile_item_off, item_hyp, n_hyp, item_cap, h_spec,
       h_maxfz, h_lo, h_hi, win_off, cnt_cap, pk_off, pk_mass, cnt, status, pk_int, tic, isum,
       reinterpret_cast<const uint2*>(pk_keys), pk_filt, n_kz > 0 ? n_kz : 0, kstride, hits);
@@ -317,7 +337,8 @@ int vk_k1_tiles(const vk_tindex* ix, const vk_frag_params* fp, float tol_lo, flo
                 int32_t* status, const float* pk_int, const float* tic, uint32_t* isum, const uint32_t* pk_keys,
                 const uint32_t* pk_filt, int n_kz, int64_t kstride, void* stream) {
   if (!cnt) return VK_E_ARG;
-  return k1_tiles_launch<false>(ix, fp, tol_lo, tol_hi, warps, tile_item_off, item_hyp, n_hyp, item_cap, h_spec,
+  const auto launch = isum ? k1_tiles_launch<false, true> : k1_tiles_launch<false, false>;
+  return launch(ix, fp, tol_lo, tol_hi, warps, tile_item_off, item_hyp, n_hyp, item_cap, h_spec,
                                 h_maxfz, h_lo, h_hi, win_off, cnt_cap, pk_off, pk_mass, cnt, status, pk_int, tic, isum,
                                 pk_keys, pk_filt, n_kz, kstride, K1Hits{}, stream);
 }
@@ -333,7 +354,8 @@ int vk_k1_hits(const vk_tindex* ix, const vk_frag_params* fp, float tol_lo, floa
   if ((hit_isum != nullptr) != (pk_int != nullptr)) return VK_E_ARG;
   K1Hits hits{thr, h_thr, hit_rc, hit_isum, seg_cnt, hyp_shift, hyp_scored,
               reinterpret_cast<unsigned long long*>(hyp_matched)};
-  return k1_tiles_launch<true>(ix, fp, tol_lo, tol_hi, warps, tile_item_off, item_hyp, n_hyp, item_cap, h_spec,
+  const auto launch = hit_isum ? k1_tiles_launch<true, true> : k1_tiles_launch<true, false>;
+  return launch(ix, fp, tol_lo, tol_hi, warps, tile_item_off, item_hyp, n_hyp, item_cap, h_spec,
                                h_maxfz, h_lo, h_hi, win_off, cnt_cap, pk_off, pk_mass, nullptr, status, pk_int, tic,
                                hit_isum, pk_keys, pk_filt, n_kz, kstride, hits, stream);
 }

@@ -11,13 +11,9 @@
 #pragma once
 #include "common.cuh"
 
-#ifndef K1_BM_LOG
-#define K1_BM_LOG 6            // log2 of the presence-bitmap bits per coarse bin (6 or 7)
-#endif
-static_assert(K1_BM_LOG == 6 || K1_BM_LOG == 7, "64 or 128 bitmap bits per coarse bin");
-
 namespace vk {
 
+constexpr int K1_BM_LOG = 6;                         // log2 of the presence-bitmap bits per coarse bin
 constexpr int K1_BM_WORDS = (1 << K1_BM_LOG) / 32;   // u32 words of a coarse bin's bitmap
 
 // cnt[hoff + l] is the count of tile row l (rows rlo <= l < rhi only).  With isum != nullptr, every match also adds
@@ -106,37 +102,18 @@ __device__ __forceinline__ uint32_t k1_bm_pos(uint32_t k, int low_bits, int bshi
   return ((k >> low_bits) << K1_BM_LOG) | ((k & ((1u << low_bits) - 1u)) >> bshift);
 }
 
-// One thread per coarse bin builds the bin's K1_BM_WORDS words in registers (the index build calls this per tile).
+// One thread per coarse bin builds the bin's 64 bits in a register (the index build calls this per tile).
 __device__ __forceinline__ void k1_build_bitmap(const uint32_t* post, const uint16_t* cb, int nb, int bits,
                                                 uint32_t* bm) {
   const int top = 32 - bits;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    unsigned long long lo = 0ull, hi = 0ull;
+    unsigned long long v = 0ull;
     const int e1 = cb[b + 1];
-    for (int e = cb[b]; e < e1; ++e) {
-      const uint32_t s = post[e] >> top;
-      if (s < 64u) lo |= 1ull << s; else hi |= 1ull << (s - 64u);
-    }
+    for (int e = cb[b]; e < e1; ++e) v |= 1ull << (post[e] >> top);
     uint32_t* w = bm + (size_t)b * K1_BM_WORDS;
-    w[0] = (uint32_t)lo;
-    w[1] = (uint32_t)(lo >> 32);
-    if (K1_BM_WORDS == 4) {
-      w[2] = (uint32_t)hi;
-      w[3] = (uint32_t)(hi >> 32);
-    }
+    w[0] = (uint32_t)v;
+    w[1] = (uint32_t)(v >> 32);
   }
-}
-
-// true when a bit in [ga, gb] (ga <= gb) is set
-__device__ __forceinline__ bool k1_bm_any(const uint32_t* bm, uint32_t ga, uint32_t gb) {
-  const uint32_t w0 = ga >> 5, w1 = gb >> 5;
-  const uint32_t head = bm[w0] & (0xffffffffu << (ga & 31u));
-  const uint32_t tail_mask = 0xffffffffu >> (31u - (gb & 31u));
-  if (w0 == w1) return (head & tail_mask) != 0u;
-  if (head) return true;
-  for (uint32_t w = w0 + 1; w < w1; ++w)
-    if (bm[w]) return true;
-  return (bm[w1] & tail_mask) != 0u;
 }
 
 // Filter word of window [ka, kb]: the bitmap position of ka in bits 0..19 and the span to kb's position in bits
@@ -150,107 +127,128 @@ __device__ __forceinline__ uint32_t k1_filter_word(uint2 k, const vk_tindex& ix)
   return ga | (min(gb - ga, 4095u) << 20);
 }
 
-// true when the window of filter word f may hold a posting of the tile with bitmap bm
-__device__ __forceinline__ bool k1_filter_pass(const uint32_t* bm, uint32_t f) {
-  if (f == K1_NO_WINDOW) return false;
-  const uint32_t ga = f & 0xfffffu, d = f >> 20;
-  if (d == 4095u) return true;
-  const uint32_t s = ga & 31u;
-  if (s + d < 32u) return ((bm[ga >> 5] >> s) & ((2u << d) - 1u)) != 0u;
-  return k1_bm_any(bm, ga, ga + d);
+// true when the window of filter word f may hold a posting of the tile with bitmap bm (bm_mask + 1 words, a power of
+// two, and one readable word behind them).  Branch-free: the window's bits lie in two neighbouring words, whichever
+// side of a word edge they start on (a tenth of the windows straddle one, so some lane of nearly every warp does);
+// windows of more than 32 bits go to the exact search.
+__device__ __forceinline__ bool k1_filter_pass(const uint32_t* bm, uint32_t bm_mask, uint32_t f) {
+  const uint32_t d = f >> 20, w = (f >> 5) & bm_mask;
+  const uint32_t v = __funnelshift_r(bm[w], bm[w + 1], f);   // from the window's first bit on
+  return f != K1_NO_WINDOW && (d >= 32u || (v & ~(0xfffffffeu << (d & 31u))) != 0u);
 }
 
-// Count the postings with key in [ka, kb] whose row lies in [rlo, rhi) (one lane, one window).
+// Count the postings with key in [ka, kb] whose row lies in [rlo, rlo + rows) (one lane, one window): one lower bound in
+// the first coarse bin, then one scan to the end of the last bin, in which a posting above the window ends it.
+template <bool ISUM>
 __device__ __forceinline__ void k1_count_range(const uint32_t* post, const uint16_t* cb, uint32_t* hw, uint32_t* iw,
-                                               int rlo, int rhi, uint32_t ka, uint32_t kb, uint32_t wgt,
-                                               const vk_tindex& ix) {
-  const int row_bits = ix.row_bits;
-  const uint32_t rowmask = (1u << row_bits) - 1u;
-  const int low_bits = ix.mass_bits - ix.cbin_bits;
-  const uint32_t lowmask = (1u << low_bits) - 1u;
+                                               int rlo, uint32_t rows, uint32_t ka, uint32_t kb, uint32_t wgt,
+                                               int row_bits, int low_bits) {
+  const uint32_t rowmask = (1u << row_bits) - 1u, lowmask = (1u << low_bits) - 1u;
   const uint32_t ba = ka >> low_bits, bb = kb >> low_bits;
-  for (uint32_t bin = ba; bin <= bb; ++bin) {
-    const uint32_t lo_key = bin == ba ? (ka & lowmask) << row_bits : 0u;
-    const uint32_t hi_key = bin == bb ? ((kb & lowmask) << row_bits) | rowmask : 0xffffffffu;
-    int e = cb[bin];
-    const int e1 = cb[bin + 1];
-    int R = e1;
-    while (e < R) {
-      const int M = (e + R) >> 1;
-      if (post[M] < lo_key) e = M + 1; else R = M;
+  const uint32_t lo_key = (ka & lowmask) << row_bits, hi_key = ((kb & lowmask) << row_bits) | rowmask;
+  int e = cb[ba], end = cb[ba + 1], last = 0;   // postings from `last` on are in the window's last bin
+  for (int span = end - e; span > 0;) {
+    const int half = span >> 1;
+    if (post[e + half] < lo_key) {
+      e += half + 1;
+      span -= half + 1;
+    } else {
+      span = half;
     }
-    for (; e < e1; ++e) {
-      const uint32_t v = post[e];
-      if (v > hi_key) break;
-      const int l = (int)(v & rowmask);
-      if (l >= rlo && l < rhi) {
-        atomicAdd(&hw[l], 1u);
-        if (iw) atomicAdd(&iw[l], wgt);
-      }
+  }
+  if (bb != ba) {
+    last = cb[bb];
+    end = cb[bb + 1];
+  }
+  for (; e < end; ++e) {
+    const uint32_t v = post[e];
+    if (v > hi_key && e >= last) break;
+    const uint32_t l = v & rowmask;
+    if (l - (uint32_t)rlo < rows) {
+      atomicAdd(&hw[l], 1u);
+      if (ISUM) atomicAdd(&iw[l], wgt);
     }
   }
 }
 
-constexpr int K1_QUEUE = 64;   // u32 entries per warp queue: (charge - 1) << 16 | peak index in the spectrum
-#ifndef K1_UNROLL
-#define K1_UNROLL 2            // filter-word loads in flight per lane
-#endif
+constexpr int K1_AHEAD = 2;    // filter words per lane tested at once, and as many more in flight
+constexpr int K1_QUEUE = 32 * (K1_AHEAD + 1);   // u32 entries per warp: (charge - 1) << 16 | peak index
+
+// A warp's next filter words: the first 32 * K1_AHEAD of an item are loaded while the item before it is worked on.
+struct K1Words {
+  uint32_t f[K1_AHEAD];
+  // words [base, base + 32 * K1_AHEAD) of an item of n; src: the item's first word plus the lane
+  __device__ __forceinline__ void load(const uint32_t* __restrict__ src, int n, int base, int lane) {
+#pragma unroll
+    for (int u = 0; u < K1_AHEAD; ++u) f[u] = base + 32 * u + lane < n ? __ldg(src + base + 32 * u) : K1_NO_WINDOW;
+  }
+};
 
 // One (tile, hypothesis) item by one warp.  For fragment charges z <= n_kz, keys[(z - 1) * kstride + p] holds the
 // window keys of peak p and filt[...] its filter word; higher charges are computed here.  q: this warp's queue.
+// words: the item's first charge-1 filter words (n_kz >= 1); on return the next item's (next_n peaks from next_p0).
+template <bool ISUM>
 __device__ __forceinline__ void k1_item_filtered(const uint32_t* post, const uint16_t* cb, const uint32_t* bm,
-                                                 uint32_t* hw, uint32_t* iw, int rlo, int rhi, int64_t p0,
-                                                 int64_t p1, int maxfz, const uint2* __restrict__ keys,
+                                                 uint32_t bm_mask, uint32_t* hw, uint32_t* iw, int rlo, int rhi,
+                                                 int64_t p0, int n, int maxfz, const uint2* __restrict__ keys,
                                                  const uint32_t* __restrict__ filt, int n_kz, int64_t kstride,
-                                                 const float* pk_mass, float tol_lo, float tol_hi, int tol_da,
-                                                 const vk_tindex& ix, int lane, uint32_t* q, const float* pk_int,
-                                                 float wscale) {
-  const int n = (int)(p1 - p0);
+                                                 const float* __restrict__ pk_mass, float tol_lo, float tol_hi,
+                                                 int tol_da, const vk_tindex& ix, int lane, uint32_t* q,
+                                                 const float* __restrict__ pk_int, float wscale, K1Words& words,
+                                                 int64_t next_p0, int next_n) {
+  const int row_bits = ix.row_bits, low_bits = ix.mass_bits - ix.cbin_bits;
+  const unsigned lt = (1u << lane) - 1u;
   int nq = 0;
   auto search = [&](uint32_t e) {
     const int zi = (int)(e >> 16);
     const int64_t p = p0 + (e & 0xffffu);
-    const uint2 k = zi < n_kz ? keys[(int64_t)zi * kstride + p]
+    const uint2 k = zi < n_kz ? __ldg(keys + (int64_t)zi * kstride + p)
                               : k1_window_keys(pk_mass[p], zi + 1, tol_lo, tol_hi, tol_da, ix);
-    const uint32_t wgt = iw ? __float2uint_rn(__fmul_rn(pk_int[p], wscale)) : 0u;
-    k1_count_range(post, cb, hw, iw, rlo, rhi, k.x, k.y, wgt, ix);
+    const uint32_t wgt = ISUM ? __float2uint_rn(__fmul_rn(__ldg(pk_int + p), wscale)) : 0u;
+    k1_count_range<ISUM>(post, cb, hw, iw, rlo, (uint32_t)(rhi - rlo), k.x, k.y, wgt, row_bits, low_bits);
   };
-  auto push = [&](bool pass, uint32_t e) {
-    const unsigned bal = __ballot_sync(0xffffffffu, pass);
-    if (pass) q[nq + __popc(bal & ((1u << lane) - 1u))] = e;
-    nq += __popc(bal);
-    if (nq >= 32) {
+  auto test = [&](const K1Words& w, uint32_t tag) {   // tag: charge and this lane's first peak
+#pragma unroll
+    for (int u = 0; u < K1_AHEAD; ++u) {
+      const bool pass = k1_filter_pass(bm, bm_mask, w.f[u]);
+      const unsigned bal = __ballot_sync(0xffffffffu, pass);
+      if (pass) q[nq + __popc(bal & lt)] = tag + 32u * u;
+      nq += __popc(bal);
+    }
+    if (nq >= 32) {   // full rounds of 32 from the end; the rest stays in front
       __syncwarp();
-      search(q[lane]);
+      do {
+        nq -= 32;
+        search(q[nq + lane]);
+      } while (nq >= 32);
       __syncwarp();
-      if (lane < nq - 32) q[lane] = q[lane + 32];
-      __syncwarp();
-      nq -= 32;
     }
   };
   for (int z = 1; z < maxfz; ++z) {
-    const uint32_t zt = (uint32_t)(z - 1) << 16;
+    const uint32_t zt = ((uint32_t)(z - 1) << 16) + (uint32_t)lane;
+    K1Words cur;
     if (z <= n_kz) {
-      const uint32_t* __restrict__ fz = filt + (int64_t)(z - 1) * kstride + p0;
-      for (int base = 0; base < n; base += 32 * K1_UNROLL) {
-        uint32_t f[K1_UNROLL];
-#pragma unroll
-        for (int u = 0; u < K1_UNROLL; ++u) {   // the loads first: K1_UNROLL in flight per lane
-          const int i = base + 32 * u + lane;
-          f[u] = i < n ? __ldg(fz + i) : K1_NO_WINDOW;
-        }
-#pragma unroll
-        for (int u = 0; u < K1_UNROLL; ++u) push(k1_filter_pass(bm, f[u]), zt | (uint32_t)(base + 32 * u + lane));
+      const uint32_t* __restrict__ src = filt + (int64_t)(z - 1) * kstride + p0 + lane;
+      if (z == 1) cur = words; else cur.load(src, n, 0, lane);
+      for (int base = 0; base < n; base += 32 * K1_AHEAD) {
+        K1Words nx;
+        nx.load(src, n, base + 32 * K1_AHEAD, lane);
+        test(cur, zt + base);
+        cur = nx;
       }
     } else {
-      for (int base = 0; base < n; base += 32) {
-        const int i = base + lane;
-        const uint32_t f = i < n ? k1_filter_word(k1_window_keys(pk_mass[p0 + i], z, tol_lo, tol_hi, tol_da, ix), ix)
-                                 : K1_NO_WINDOW;
-        push(k1_filter_pass(bm, f), zt | (uint32_t)i);
+      for (int base = 0; base < n; base += 32 * K1_AHEAD) {
+#pragma unroll
+        for (int u = 0; u < K1_AHEAD; ++u) {
+          const int i = base + 32 * u + lane;
+          cur.f[u] = i < n ? k1_filter_word(k1_window_keys(pk_mass[p0 + i], z, tol_lo, tol_hi, tol_da, ix), ix)
+                           : K1_NO_WINDOW;
+        }
+        test(cur, zt + base);
       }
     }
   }
+  if (n_kz > 0) words.load(filt + next_p0 + lane, next_n, 0, lane);
   __syncwarp();
   if (lane < nq) search(q[lane]);
 }
