@@ -137,8 +137,8 @@ __device__ __forceinline__ bool k1_filter_pass(const uint32_t* bm, uint32_t bm_m
   return f != K1_NO_WINDOW && (d >= 32u || (v & ~(0xfffffffeu << (d & 31u))) != 0u);
 }
 
-// Count the postings with key in [ka, kb] whose row lies in [rlo, rlo + rows) (one lane, one window): one lower bound in
-// the first coarse bin, then one scan to the end of the last bin, in which a posting above the window ends it.
+// Count the postings with key in [ka, kb] whose row lies in [rlo, rlo + rows) (one lane, one window): one lower bound
+// in the first coarse bin, then one scan to the end of the last bin, in which a posting above the window ends it.
 template <bool ISUM>
 __device__ __forceinline__ void k1_count_range(const uint32_t* post, const uint16_t* cb, uint32_t* hw, uint32_t* iw,
                                                int rlo, uint32_t rows, uint32_t ka, uint32_t kb, uint32_t wgt,

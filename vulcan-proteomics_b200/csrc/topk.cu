@@ -143,9 +143,9 @@ __device__ __forceinline__ int64_t win_rows(int64_t w0, int64_t lo, int64_t hi, 
 // before -> now: 40,000 spectra at topk 100 0.725 -> 0.203 ms, 16,384 with 2,100 window rows each at topk 200
 // 1.588 -> 0.178, 10,001 at topk 500 1.112 -> 0.113, 32 spectra 0.009 -> 0.0064 (and 0.002 for the launch that looks
 // for what was left over).  Staging the rows of step 4 in shared memory for whole-sector writes was slower (0.228 and
-// 0.142: fewer warps per SM), and so was a tally in byte fields of registers (0.216).  What does not fit goes to select_topk_k by n_cand = -1: more than 32
-// hypotheses or overlapping windows, more than TR_WORDS * 32 window rows, a count above 254, a partner outside its
-// own hypothesis' window.
+// 0.142: fewer warps per SM), and so was a tally in byte fields of registers (0.216).
+// What does not fit goes to select_topk_k by n_cand = -1: more than 32 hypotheses or overlapping windows, more than
+// TR_WORDS * 32 window rows, a count above 254, a partner outside its own hypothesis' window.
 constexpr int TR_WORDS = 384;        // bitmap words per spectrum: 12,288 window rows
 constexpr int TR_TOPK = 512;         // longest list
 
@@ -362,7 +362,8 @@ select_topk_rows_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
 // ------------------------------------------------------------------------------------------ any windows
 // One spectrum per warp; rest: only the spectra select_topk_rows_k left (n_cand = -1).
 __global__ void __launch_bounds__(TK_WARPS * 32)
-select_topk_k(int n_spec, int rest, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi, const int64_t* win_off,
+select_topk_k(int n_spec, int rest, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
+              const int64_t* win_off,
               const int32_t* cnt, int64_t cnt_cap, const int64_t* partner, int thr, int topk, int pair_closure, int cap,
               int list_pow2, int key_cap, int64_t* c_hyp, int64_t* c_row, int64_t* c_cnt, int64_t* n_cand,
               uint32_t* hyp_scored, uint64_t* hyp_matched, int64_t* spec_scored, int64_t* spec_matched) {
@@ -552,11 +553,17 @@ struct HitScratch {
 // (one per tile a window covers; a hypothesis with tile shift 0 ran no item and has none) in hypothesis order, tile
 // order, and each segment's hits in row order.  Two parallel rounds per 32 segments: their hit counts (seg_cnt at
 // the segment's first slot), then the hits themselves spread over the lanes.  f(ok, slot, value, local hypothesis)
-// is called by the whole warp; lanes with ok hold a hit.
-template <class F>
+// is called by the whole warp; lanes with ok hold a hit.  more(): false (the same in every lane) ends the visit before
+// the next 32 segments.  part, parts: this warp's share of each group's hits.
+struct AllHits {
+  __device__ __forceinline__ bool operator()() const { return true; }
+};
+
+template <class F, class G = AllHits>
 __device__ __forceinline__ void gather_hits(HitScratch& S, int nv, int64_t hb, const int64_t* h_lo, const int64_t* h_hi,
                                             const int64_t* win_off, const int8_t* hyp_shift, const uint32_t* seg_cnt,
-                                            const uint64_t* rc, int lane, F&& f) {
+                                            const uint64_t* rc, int lane, F&& f, G&& more = G(), int part = 0,
+                                            int parts = 1) {
   int nt = 0;
   if (lane < nv) {
     const int64_t h = hb + S.hyp[lane];
@@ -576,7 +583,7 @@ __device__ __forceinline__ void gather_hits(HitScratch& S, int nv, int64_t hb, c
   S.seg_base[lane] = incl - nt;
   const int total = __shfl_sync(VK_FULL, incl, 31);
   __syncwarp();
-  for (int k0 = 0; k0 < total; k0 += 32) {
+  for (int k0 = 0; k0 < total && more(); k0 += 32) {
     const int k = k0 + lane;
     uint32_t c = 0;
     int64_t slot = 0;
@@ -601,7 +608,7 @@ __device__ __forceinline__ void gather_hits(HitScratch& S, int nv, int64_t hb, c
     S.pos[lane] = pincl - (int)c;
     S.who[lane] = who;
     __syncwarp();
-    for (int u0 = 0; u0 < n_hits; u0 += 32) {
+    for (int u0 = part * 32; u0 < n_hits; u0 += parts * 32) {
       const int u = u0 + lane;
       const bool ok = u < n_hits;
       int64_t at = 0;
@@ -626,181 +633,14 @@ __device__ __forceinline__ void gather_hits(HitScratch& S, int nv, int64_t hb, c
 __device__ __forceinline__ int hit_count(uint64_t v) { return (int)min(v >> 32, (uint64_t)INT32_MAX); }
 __device__ __forceinline__ int64_t hit_row(uint64_t v) { return (int64_t)(uint32_t)v; }
 
-// Shortlist from the hit lists of vk_k1_hits, one warp per spectrum: the hits of the spectrum's hypotheses ranked by
-// (count desc, row desc, hypothesis asc) with the keys of select_topk_k, the first topk kept (all when fewer),
-// optionally with pair closure, sorted by (row, hypothesis), duplicate rows merged to the lowest hypothesis (its
-// intensity sum) and the highest count: the slots select_topk_k writes, plus c_isum.
-//   Fast path (no closure, at most 32 hypotheses, their windows pairwise disjoint -- the usual case): the hypotheses
-//   are visited in window order and each one's hits come in row order, so the collected hits are already sorted by
-//   row with no duplicates; selection keeps that order and no sort is needed.
-//   Otherwise: collect, select, add partners, bitonic sort and merge.  Spectra with more hits than shared memory
-//   holds run the radix select over the hit lists in global memory and a second read.
-__global__ void __launch_bounds__(TK_WARPS * 32)
-select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
-              const int64_t* win_off, const int8_t* hyp_shift, const uint32_t* seg_cnt, const uint64_t* rc,
-              const uint32_t* hit_isum,
-              const uint32_t* hyp_scored, const uint64_t* hyp_matched, int topk, int pair_closure,
-              const int64_t* partner, int cap, int list_pow2, int key_cap, int64_t* c_hyp, int64_t* c_row,
-              int64_t* c_cnt, uint32_t* c_isum, int64_t* n_cand, int64_t* spec_scored, int64_t* spec_matched) {
-  extern __shared__ __align__(16) uint8_t tk_smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int s = blockIdx.x * TK_WARPS + warp;
-  if (s >= n_spec) return;
-  const size_t per_warp = (size_t)key_cap * 12 + (size_t)list_pow2 * 16 + 256 * 4 + sizeof(HitScratch);
-  uint8_t* base = tk_smem + per_warp * warp;
-  HitScratch& S = *reinterpret_cast<HitScratch*>(base + per_warp - sizeof(HitScratch));
-  uint64_t* key = reinterpret_cast<uint64_t*>(base);
-  uint32_t* src = reinterpret_cast<uint32_t*>(base + (size_t)key_cap * 8);   // hit slot - win_off[hb]
-  int32_t* row = reinterpret_cast<int32_t*>(src + key_cap);
-  int32_t* hl = row + list_pow2;
-  int32_t* cnt = hl + list_pow2;
-  uint32_t* isum = reinterpret_cast<uint32_t*>(cnt + list_pow2);
-  uint32_t* hist = isum + list_pow2;
+// The kept hits of spectrum s (n_sel rows in row / hl / cnt / isum, in any order) to its slots, by one warp: closure
+// partners, sort by (row, hypothesis), duplicate rows merged.  key: room for the next power of two of the list.
+__device__ __forceinline__ void finish_hits(int lane, int s, int64_t hb, int n_sel, int pair_closure,
+                                            const int64_t* partner, int cap, uint64_t* key, int32_t* row, int32_t* hl,
+                                            int32_t* cnt, uint32_t* isum, int64_t* c_hyp, int64_t* c_row,
+                                            int64_t* c_cnt, uint32_t* c_isum, int64_t* n_cand) {
   const unsigned lt_mask = (1u << lane) - 1u;
-  const int64_t hb = spec_hyp_off[s], he = spec_hyp_off[s + 1];
-  const int nhs = (int)(he - hb);
-  const int64_t w_base = he > hb ? win_off[hb] : 0;
   const int64_t slot = (int64_t)s * cap;
-  // per-spectrum statistics from K1's per-hypothesis totals
-  long long sc = 0, mt = 0;
-  for (int64_t h = hb + lane; h < he; h += 32) {
-    sc += hyp_scored[h];
-    mt += (long long)hyp_matched[h];
-  }
-  sc = vk::warp_sum(sc);
-  mt = vk::warp_sum(mt);
-  if (lane == 0 && spec_scored) {
-    spec_scored[s] = sc;
-    spec_matched[s] = mt;
-  }
-  // every hit of the spectrum's hypotheses in index order, 32 hypotheses at a time
-  auto visit_all = [&](auto&& f) {
-    for (int g0 = 0; g0 < nhs; g0 += 32) {
-      __syncwarp();
-      if (lane < min(32, nhs - g0)) S.hyp[lane] = g0 + lane;
-      __syncwarp();
-      gather_hits(S, min(32, nhs - g0), hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane, f);
-    }
-  };
-
-  // ---------------------------------------------------------------- fast path
-  bool fast = !pair_closure && nhs <= 32;
-  int my_rank = 0;
-  if (fast) {
-    const bool mine = lane < nhs;
-    const int64_t my_lo = mine ? h_lo[hb + lane] : 0, my_hi = mine ? h_hi[hb + lane] : 0;
-    const bool live = mine && my_hi > my_lo;
-    bool overlap = false;
-    for (int j = 0; j < nhs; ++j) {
-      const int64_t lo_j = __shfl_sync(VK_FULL, my_lo, j), hi_j = __shfl_sync(VK_FULL, my_hi, j);
-      const bool live_j = hi_j > lo_j;
-      if (live && live_j && j != lane) {
-        if (lo_j < my_lo || (lo_j == my_lo && j < lane)) ++my_rank;
-        overlap |= lo_j < my_hi && my_lo < hi_j;
-      }
-      if (mine && !live && live_j) ++my_rank;   // empty windows after every live one
-      if (mine && !live && !live_j && j < lane) ++my_rank;
-    }
-    fast = !__any_sync(VK_FULL, overlap);
-  }
-  if (fast) {
-    long long n_app = 0;
-    __syncwarp();
-    if (lane < nhs) S.hyp[my_rank] = lane;     // the hypotheses in window order
-    __syncwarp();
-    gather_hits(S, nhs, hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane,
-                [&](bool ok, int64_t pos, uint64_t v, int hl_) {
-      const unsigned m = __ballot_sync(VK_FULL, ok);
-      const long long at = n_app + __popc(m & lt_mask);
-      if (ok && at < key_cap) {
-        key[at] = sel_key(hit_count(v), hit_row(v), hl_);
-        src[at] = (uint32_t)(pos - w_base);
-      }
-      n_app += __popc(m);
-    });
-    __syncwarp();
-    if (n_app <= key_cap) {
-      const int n_k = (int)n_app;
-      const bool limit = n_k > topk;
-      const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, hist, lane) : 0ull;
-      int n_out = 0;
-      for (int i0 = 0; i0 < n_k; i0 += 32) {
-        const int i = i0 + lane;
-        const uint64_t k = i < n_k ? key[i] : 0ull;
-        const bool take = i < n_k && (!limit || k >= kth);
-        const unsigned m = __ballot_sync(VK_FULL, take);
-        if (take) {
-          const int64_t pos = w_base + src[i];
-          const uint64_t v = rc[pos];
-          const int64_t at = slot + n_out + __popc(m & lt_mask);
-          c_hyp[at] = hb + ((1 << 18) - 1 - (int)(k & 0x3ffff));
-          c_row[at] = hit_row(v);
-          c_cnt[at] = hit_count(v);
-          if (c_isum) c_isum[at] = hit_isum[pos];
-        }
-        n_out += __popc(m);
-      }
-      if (lane == 0) n_cand[s] = n_out;
-      return;
-    }
-  }
-
-  // ---------------------------------------------------------------- general path
-  long long n_app = 0;
-  visit_all([&](bool ok, int64_t pos, uint64_t v, int hl_) {
-    const unsigned m = __ballot_sync(VK_FULL, ok);
-    const long long at = n_app + __popc(m & lt_mask);
-    if (ok && at < key_cap) {
-      key[at] = sel_key(hit_count(v), hit_row(v), hl_);
-      src[at] = (uint32_t)(pos - w_base);
-    }
-    n_app += __popc(m);
-  });
-  __syncwarp();
-  const bool limit = n_app > topk;
-  int n_sel = 0;
-  auto take_hit = [&](bool take, int64_t pos_g, int h_local) {
-    const unsigned m = __ballot_sync(VK_FULL, take);
-    if (take) {
-      const int at = n_sel + __popc(m & lt_mask);
-      const uint64_t v = rc[pos_g];
-      row[at] = (int32_t)hit_row(v);
-      hl[at] = h_local;
-      cnt[at] = hit_count(v);
-      isum[at] = hit_isum ? hit_isum[pos_g] : 0u;
-    }
-    n_sel += __popc(m);
-  };
-  if (n_app <= key_cap) {
-    const int n_k = (int)n_app;
-    const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, hist, lane) : 0ull;
-    for (int i0 = 0; i0 < n_k; i0 += 32) {
-      const int i = i0 + lane;
-      const uint64_t k = i < n_k ? key[i] : 0ull;
-      const bool take = i < n_k && (!limit || k >= kth);
-      take_hit(take, take ? w_base + src[i] : 0, (1 << 18) - 1 - (int)(k & 0x3ffff));
-    }
-  } else {
-    uint64_t prefix = 0, pmask = 0;
-    long long need = topk;
-    for (int shift = 56; shift >= 0; shift -= 8) {
-      for (int i = lane; i < 256; i += 32) hist[i] = 0;
-      __syncwarp();
-      visit_all([&](bool ok, int64_t, uint64_t v, int hl_) {
-        if (!ok) return;
-        const uint64_t k = sel_key(hit_count(v), hit_row(v), hl_);
-        if ((k & pmask) == prefix) atomicAdd(&hist[(k >> shift) & 255], 1u);
-      });
-      __syncwarp();
-      prefix |= (uint64_t)radix_digit(hist, need, lane) << shift;
-      pmask |= 255ull << shift;
-      __syncwarp();
-    }
-    visit_all([&](bool ok, int64_t pos, uint64_t v, int hl_) {
-      const bool take = ok && sel_key(hit_count(v), hit_row(v), hl_) >= prefix;
-      take_hit(take, pos, hl_);
-    });
-  }
   __syncwarp();
   // pair closure: the partner row of every kept hit, same hypothesis, count -1 (no intensity sum)
   int n_list = n_sel;
@@ -844,6 +684,365 @@ select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, cons
     n_out += __popc(m);
   }
   if (lane == 0) n_cand[s] = n_out;
+}
+
+// Shortlist from the hit lists of vk_k1_hits, one warp per spectrum: the hits of the spectrum's hypotheses ranked by
+// (count desc, row desc, hypothesis asc) with the keys of select_topk_k, the first topk kept (all when fewer),
+// optionally with pair closure, sorted by (row, hypothesis), duplicate rows merged to the lowest hypothesis (its
+// intensity sum) and the highest count: the slots select_topk_k writes, plus c_isum.
+//   Fast path (no closure, at most 32 hypotheses, their windows pairwise disjoint -- the usual case): the hypotheses
+//   are visited in window order and each one's hits come in row order, so the collected hits are already sorted by
+//   row with no duplicates; selection keeps that order and no sort is needed.
+//   Otherwise: collect, select, add partners, bitonic sort and merge.  Spectra with more hits than shared memory
+//   holds are left to select_hits_big_k (n_cand = -1), as soon as that is seen.
+__global__ void __launch_bounds__(TK_WARPS * 32)
+select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
+              const int64_t* win_off, const int8_t* hyp_shift, const uint32_t* seg_cnt, const uint64_t* rc,
+              const uint32_t* hit_isum,
+              const uint32_t* hyp_scored, const uint64_t* hyp_matched, int topk, int pair_closure,
+              const int64_t* partner, int cap, int list_pow2, int key_cap, int64_t* c_hyp, int64_t* c_row,
+              int64_t* c_cnt, uint32_t* c_isum, int64_t* n_cand, int64_t* spec_scored, int64_t* spec_matched) {
+  extern __shared__ __align__(16) uint8_t tk_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s = blockIdx.x * TK_WARPS + warp;
+  if (s >= n_spec) return;
+  const size_t per_warp = (size_t)key_cap * 12 + (size_t)list_pow2 * 16 + 256 * 4 + sizeof(HitScratch);
+  uint8_t* base = tk_smem + per_warp * warp;
+  HitScratch& S = *reinterpret_cast<HitScratch*>(base + per_warp - sizeof(HitScratch));
+  uint64_t* key = reinterpret_cast<uint64_t*>(base);
+  uint32_t* src = reinterpret_cast<uint32_t*>(base + (size_t)key_cap * 8);   // hit slot - win_off[hb]
+  int32_t* row = reinterpret_cast<int32_t*>(src + key_cap);
+  int32_t* hl = row + list_pow2;
+  int32_t* cnt = hl + list_pow2;
+  uint32_t* isum = reinterpret_cast<uint32_t*>(cnt + list_pow2);
+  uint32_t* hist = isum + list_pow2;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const int64_t hb = spec_hyp_off[s], he = spec_hyp_off[s + 1];
+  const int nhs = (int)(he - hb);
+  const int64_t w_base = he > hb ? win_off[hb] : 0;
+  const int64_t slot = (int64_t)s * cap;
+  // per-spectrum statistics from K1's per-hypothesis totals
+  long long sc = 0, mt = 0;
+  for (int64_t h = hb + lane; h < he; h += 32) {
+    sc += hyp_scored[h];
+    mt += (long long)hyp_matched[h];
+  }
+  sc = vk::warp_sum(sc);
+  mt = vk::warp_sum(mt);
+  if (lane == 0 && spec_scored) {
+    spec_scored[s] = sc;
+    spec_matched[s] = mt;
+  }
+  // ---------------------------------------------------------------- fast path
+  bool fast = !pair_closure && nhs <= 32;
+  int my_rank = 0;
+  if (fast) {
+    const bool mine = lane < nhs;
+    const int64_t my_lo = mine ? h_lo[hb + lane] : 0, my_hi = mine ? h_hi[hb + lane] : 0;
+    const bool live = mine && my_hi > my_lo;
+    bool overlap = false;
+    for (int j = 0; j < nhs; ++j) {
+      const int64_t lo_j = __shfl_sync(VK_FULL, my_lo, j), hi_j = __shfl_sync(VK_FULL, my_hi, j);
+      const bool live_j = hi_j > lo_j;
+      if (live && live_j && j != lane) {
+        if (lo_j < my_lo || (lo_j == my_lo && j < lane)) ++my_rank;
+        overlap |= lo_j < my_hi && my_lo < hi_j;
+      }
+      if (mine && !live && live_j) ++my_rank;   // empty windows after every live one
+      if (mine && !live && !live_j && j < lane) ++my_rank;
+    }
+    fast = !__any_sync(VK_FULL, overlap);
+  }
+  if (fast) {
+    long long n_app = 0;
+    __syncwarp();
+    if (lane < nhs) S.hyp[my_rank] = lane;     // the hypotheses in window order
+    __syncwarp();
+    gather_hits(S, nhs, hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane,
+                [&](bool ok, int64_t pos, uint64_t v, int hl_) {
+      const unsigned m = __ballot_sync(VK_FULL, ok);
+      const long long at = n_app + __popc(m & lt_mask);
+      if (ok && at < key_cap) {
+        key[at] = sel_key(hit_count(v), hit_row(v), hl_);
+        src[at] = (uint32_t)(pos - w_base);
+      }
+      n_app += __popc(m);
+    }, [&]() { return n_app <= key_cap; });
+    __syncwarp();
+    if (n_app > key_cap) {   // more than shared memory holds: select_hits_big_k
+      if (lane == 0) n_cand[s] = -1;
+      return;
+    }
+    {
+      const int n_k = (int)n_app;
+      const bool limit = n_k > topk;
+      const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, hist, lane) : 0ull;
+      int n_out = 0;
+      for (int i0 = 0; i0 < n_k; i0 += 32) {
+        const int i = i0 + lane;
+        const uint64_t k = i < n_k ? key[i] : 0ull;
+        const bool take = i < n_k && (!limit || k >= kth);
+        const unsigned m = __ballot_sync(VK_FULL, take);
+        if (take) {
+          const int64_t pos = w_base + src[i];
+          const uint64_t v = rc[pos];
+          const int64_t at = slot + n_out + __popc(m & lt_mask);
+          c_hyp[at] = hb + ((1 << 18) - 1 - (int)(k & 0x3ffff));
+          c_row[at] = hit_row(v);
+          c_cnt[at] = hit_count(v);
+          if (c_isum) c_isum[at] = hit_isum[pos];
+        }
+        n_out += __popc(m);
+      }
+      if (lane == 0) n_cand[s] = n_out;
+      return;
+    }
+  }
+
+  // ---------------------------------------------------------------- general path
+  long long n_app = 0;
+  for (int g0 = 0; g0 < nhs && n_app <= key_cap; g0 += 32) {   // 32 hypotheses at a time, in index order
+    __syncwarp();
+    if (lane < min(32, nhs - g0)) S.hyp[lane] = g0 + lane;
+    __syncwarp();
+    gather_hits(S, min(32, nhs - g0), hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane,
+                [&](bool ok, int64_t pos, uint64_t v, int hl_) {
+      const unsigned m = __ballot_sync(VK_FULL, ok);
+      const long long at = n_app + __popc(m & lt_mask);
+      if (ok && at < key_cap) {
+        key[at] = sel_key(hit_count(v), hit_row(v), hl_);
+        src[at] = (uint32_t)(pos - w_base);
+      }
+      n_app += __popc(m);
+    }, [&]() { return n_app <= key_cap; });
+  }
+  __syncwarp();
+  if (n_app > key_cap) {   // more than shared memory holds: select_hits_big_k
+    if (lane == 0) n_cand[s] = -1;
+    return;
+  }
+  const int n_k = (int)n_app;
+  const bool limit = n_k > topk;
+  int n_sel = 0;
+  const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, hist, lane) : 0ull;
+  for (int i0 = 0; i0 < n_k; i0 += 32) {
+    const int i = i0 + lane;
+    const uint64_t k = i < n_k ? key[i] : 0ull;
+    const bool take = i < n_k && (!limit || k >= kth);
+    const unsigned m = __ballot_sync(VK_FULL, take);
+    if (take) {
+      const int at = n_sel + __popc(m & lt_mask);
+      const int64_t pos_g = w_base + src[i];
+      const uint64_t v = rc[pos_g];
+      row[at] = (int32_t)hit_row(v);
+      hl[at] = (1 << 18) - 1 - (int)(k & 0x3ffff);
+      cnt[at] = hit_count(v);
+      isum[at] = hit_isum ? hit_isum[pos_g] : 0u;
+    }
+    n_sel += __popc(m);
+  }
+  __syncwarp();
+  finish_hits(lane, s, hb, n_sel, pair_closure, partner, cap, key, row, hl, cnt, isum, c_hyp, c_row, c_cnt, c_isum,
+              n_cand);
+}
+
+// The spectra select_hits_k left (n_cand = -1; open searches, whose windows span most of the index): a CTA per
+// spectrum, its warps sharing the hits of each 32 segments.  The hits are visited three times, usually: a histogram of
+// their counts gives the count T of the topk-th hit; one of the row bins (256 equal ranges of the rows still in
+// question) of the hits tied at T gives the bin it lies in, again within that bin while too many hits tie; then the
+// hits above it are collected as keys and the exact topk-th is selected among them, and one warp finishes the list.
+// What bounds it is the latency of the dependent reads (segment count, hit) of a visit.  A warp per spectrum ran an
+// eight-pass radix select over the lists and two more visits, each some 140 us for 20,000 hits; 777 spectra with open
+// windows: 1.41 ms before, 0.22 now (0.049 of it select_hits_k); 4,000 spectra of which one in five holds more than
+// 512 hits: 0.146 before, 0.142 now.  8 and 4 warps per CTA: 0.25 and 0.31 on the open windows.  Warps that take whole
+// groups of segments instead of a share of each group's hits: 0.20, but 0.170 on the 4,000 (one group each).
+constexpr int HB_WARPS = 16;
+constexpr int HB_COUNTS = 1024;     // histogram bins of the counts; the last holds all larger ones
+
+struct BigScratch {
+  HitScratch warp[HB_WARPS];
+  uint32_t hist[HB_COUNTS];
+  int32_t todo[HB_WARPS * 32];
+  int n_todo, n_key, value, above;
+};
+
+// With hist[n] (n a multiple of 32) the numbers of keys per digit: the largest digit d with more than `most` keys at
+// or above it (-1: none), and the keys above d.  By one warp.
+__device__ __forceinline__ int top_digit(const uint32_t* hist, int n, uint32_t most, uint32_t& above, int lane) {
+  uint32_t seen = 0u;
+  for (int d0 = n - 32; d0 >= 0; d0 -= 32) {
+    const uint32_t v = hist[d0 + 31 - lane];       // lane 0: the highest digit
+    const uint32_t inc = (uint32_t)vk::warp_incl_scan_i32((int)v) + seen;
+    const unsigned over = __ballot_sync(VK_FULL, inc > most);
+    if (over) {
+      const int l = __ffs(over) - 1;
+      above = __shfl_sync(VK_FULL, inc - v, l);
+      return d0 + 31 - l;
+    }
+    seen = __shfl_sync(VK_FULL, inc, 31);
+  }
+  above = seen;
+  return -1;
+}
+
+__global__ void __launch_bounds__(HB_WARPS * 32)
+select_hits_big_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
+                  const int64_t* win_off, const int8_t* hyp_shift, const uint32_t* seg_cnt, const uint64_t* rc,
+                  const uint32_t* hit_isum, int topk, int pair_closure, const int64_t* partner, int cap, int list_pow2,
+                  int key_cap, int64_t* c_hyp, int64_t* c_row, int64_t* c_cnt, uint32_t* c_isum, int64_t* n_cand) {
+  extern __shared__ __align__(16) uint8_t tk_smem[];
+  BigScratch& B = *reinterpret_cast<BigScratch*>(tk_smem);
+  uint64_t* key = reinterpret_cast<uint64_t*>(tk_smem + ((sizeof(BigScratch) + 15) & ~(size_t)15));
+  uint32_t* src = reinterpret_cast<uint32_t*>(key + key_cap);   // hit slot - win_off[hb]
+  int32_t* row = reinterpret_cast<int32_t*>(src + key_cap);
+  int32_t* hl = row + list_pow2;
+  int32_t* cnt = hl + list_pow2;
+  uint32_t* isum = reinterpret_cast<uint32_t*>(cnt + list_pow2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  HitScratch& S = B.warp[warp];
+  for (int64_t base = blockIdx.x; base < n_spec; base += (int64_t)gridDim.x * blockDim.x) {
+    // this CTA's spectra of the round: base + t * grid for its threads t; those left over are listed
+    if (tid == 0) B.n_todo = 0;
+    __syncthreads();
+    const int64_t mine = base + (int64_t)tid * gridDim.x;
+    if (mine < n_spec && n_cand[mine] < 0) B.todo[atomicAdd(&B.n_todo, 1)] = (int32_t)mine;
+    __syncthreads();
+    for (int q = 0; q < B.n_todo; ++q) {
+      const int s = B.todo[q];
+      const int64_t hb = spec_hyp_off[s];
+      const int nhs = (int)(spec_hyp_off[s + 1] - hb);
+      const int64_t w_base = win_off[hb];
+      auto visit = [&](auto&& f) {   // the warp's share of the spectrum's hits
+        for (int g0 = 0; g0 < nhs; g0 += 32) {
+          __syncwarp();
+          if (lane < min(32, nhs - g0)) S.hyp[lane] = g0 + lane;
+          __syncwarp();
+          gather_hits(S, min(32, nhs - g0), hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane, f, AllHits(), warp,
+                      HB_WARPS);
+        }
+      };
+      auto clear = [&](int n) {
+        __syncthreads();
+        for (int i = tid; i < n; i += blockDim.x) B.hist[i] = 0u;
+        if (tid == 0) B.n_key = 0;
+        __syncthreads();
+      };
+      auto find = [&](int n, uint32_t most) {   // (value, above) of top_digit in every thread
+        __syncthreads();
+        if (warp == 0) {
+          uint32_t a;
+          const int d = top_digit(B.hist, n, most, a, lane);
+          if (lane == 0) {
+            B.value = d;
+            B.above = (int)a;
+          }
+        }
+        __syncthreads();
+      };
+      // the counts
+      clear(HB_COUNTS);
+      visit([&](bool ok, int64_t, uint64_t v, int) {
+        if (ok) atomicAdd(&B.hist[min(hit_count(v), HB_COUNTS - 1)], 1u);
+      });
+      find(HB_COUNTS, (uint32_t)topk);
+      const int T = B.value;                   // ties at T are in question; -1: at most topk hits, all taken
+      int above = B.above;
+      // the rows of the ties: [r_lo, r_hi) still in question, everything above taken
+      int64_t r_lo = 0, r_hi = 0;
+      bool all = false;
+      if (T >= 0) {
+        int64_t a = INT64_MAX, b = 0;
+        for (int h = lane; h < nhs; h += 32) {
+          const int64_t lo = h_lo[hb + h], hi = h_hi[hb + h];
+          if (hi > lo) {
+            a = min(a, lo);
+            b = max(b, hi);
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          a = min(a, __shfl_xor_sync(VK_FULL, a, o));
+          b = max(b, __shfl_xor_sync(VK_FULL, b, o));
+        }
+        r_lo = a;
+        r_hi = b;
+        int64_t left = B.hist[T];              // hits tied at T with rows in question
+        while (T < HB_COUNTS - 1 && above + left > key_cap && r_hi - r_lo > 1) {
+          const int64_t width = (r_hi - r_lo + 255) / 256;
+          clear(256);
+          visit([&](bool ok, int64_t, uint64_t v, int) {
+            const int64_t r = hit_row(v);
+            if (ok && min(hit_count(v), HB_COUNTS - 1) == T && r >= r_lo && r < r_hi)
+              atomicAdd(&B.hist[(int)((r - r_lo) / width)], 1u);
+          });
+          find(256, (uint32_t)(topk - above));
+          const int d = B.value;               // (more than topk - above hits are in question, so d >= 0)
+          above += B.above;
+          left = B.hist[d];
+          r_hi = min(r_hi, r_lo + (d + 1) * width);
+          r_lo = r_lo + d * width;
+        }
+        all = above + left > key_cap;
+      }
+      uint64_t floor = 0ull;                   // (all) the topk-th key, where counts past the histogram or more
+      if (all) {                               // hypotheses on one row than fit tie: a radix select over the keys
+        uint64_t pmask = 0ull;
+        uint32_t need = (uint32_t)topk;
+        for (int shift = 56; shift >= 0; shift -= 8) {
+          clear(256);
+          visit([&](bool ok, int64_t, uint64_t v, int hl_) {
+            const uint64_t k = sel_key(hit_count(v), hit_row(v), hl_);
+            if (ok && (k & pmask) == floor) atomicAdd(&B.hist[(k >> shift) & 255], 1u);
+          });
+          find(256, need - 1u);
+          need -= (uint32_t)B.above;
+          floor |= (uint64_t)B.value << shift;
+          pmask |= 255ull << shift;
+        }
+      }
+      // collect the keys: counts above T, and the ties from row r_lo on
+      clear(0);
+      visit([&](bool ok, int64_t pos, uint64_t v, int hl_) {
+        const int c = min(hit_count(v), HB_COUNTS - 1);
+        if (ok && (all ? sel_key(hit_count(v), hit_row(v), hl_) >= floor : c > T || (c == T && hit_row(v) >= r_lo))) {
+          const int at = atomicAdd(&B.n_key, 1);
+          if (at < key_cap) {
+            key[at] = sel_key(hit_count(v), hit_row(v), hl_);
+            src[at] = (uint32_t)(pos - w_base);
+          }
+        }
+      });
+      __syncthreads();
+      if (warp == 0) {
+        const unsigned lt_mask = (1u << lane) - 1u;
+        const int n_k = min(B.n_key, key_cap);
+        const bool limit = n_k > topk;
+        const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, B.hist, lane) : 0ull;
+        int n_sel = 0;
+        for (int i0 = 0; i0 < n_k; i0 += 32) {
+          const int i = i0 + lane;
+          const uint64_t k = i < n_k ? key[i] : 0ull;
+          const bool take = i < n_k && (!limit || k >= kth);
+          const unsigned m = __ballot_sync(VK_FULL, take);
+          if (take) {
+            const int at = n_sel + __popc(m & lt_mask);
+            const int64_t pos_g = w_base + src[i];
+            const uint64_t v = rc[pos_g];
+            row[at] = (int32_t)hit_row(v);
+            hl[at] = (1 << 18) - 1 - (int)(k & 0x3ffff);
+            cnt[at] = hit_count(v);
+            isum[at] = hit_isum ? hit_isum[pos_g] : 0u;
+          }
+          n_sel += __popc(m);
+        }
+        __syncwarp();
+        finish_hits(lane, s, hb, n_sel, pair_closure, partner, cap, key, row, hl, cnt, isum, c_hyp, c_row, c_cnt,
+                    c_isum, n_cand);
+      }
+      __syncthreads();
+    }
+    __syncthreads();
+  }
 }
 
 // select_hits_k for a short list without pair closure (topk <= 32), one warp per spectrum, with no per-warp key
@@ -1136,6 +1335,15 @@ int vk_select_hits(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
       n_spec, spec_hyp_off, h_lo, h_hi, win_off, hyp_shift, seg_cnt, hit_rc, hit_isum, hyp_scored, hyp_matched, topk,
       pair_closure, partner, cap, list_pow2, key_cap, c_hyp, c_row, c_cnt, c_isum, n_cand, spec_scored,
       spec_matched);
+  const int rc = vk_launch_status();
+  if (rc != 0) return rc;
+  const int big_cap = 2 * list_pow2 > 1024 ? 2 * list_pow2 : 1024;
+  const size_t bsh = ((sizeof(BigScratch) + 15) & ~(size_t)15) + (size_t)big_cap * 12 + (size_t)list_pow2 * 16;
+  e = cudaFuncSetAttribute(select_hits_big_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsh);
+  if (e != cudaSuccess) return vk_err(e);
+  select_hits_big_k<<<(unsigned)(n_spec < 592 ? n_spec : 592), HB_WARPS * 32, bsh, (cudaStream_t)stream>>>(
+      n_spec, spec_hyp_off, h_lo, h_hi, win_off, hyp_shift, seg_cnt, hit_rc, hit_isum, topk, pair_closure, partner, cap,
+      list_pow2, big_cap, c_hyp, c_row, c_cnt, c_isum, n_cand);
   return vk_launch_status();
 }
 

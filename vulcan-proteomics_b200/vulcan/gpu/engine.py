@@ -709,7 +709,7 @@ def _shortlist_hits(gi: GpuIndex, p: SearchParams, n: int, dh, k1h: dict, topk: 
                              K.ptr(k1h["hyp_matched"]), topk, int(closure), K.ptr(gi.partner), cap, K.ptr(s_hyp),
                              K.ptr(s_row), K.ptr(s_cnt),
                              K.ptr(s_isum) if isum else None, K.ptr(n_cand), K.ptr(spec_scored),
-                             K.ptr(spec_matched), K.stream()), "select_hits")
+                             K.ptr(spec_matched), K.stream()), "select_hits", 1 if topk <= 32 and not closure else 2)
     cand_off = _scan(n_cand[:n])
     c_hyp = torch.empty_like(s_hyp)
     c_row = torch.empty_like(s_hyp)
