@@ -113,7 +113,7 @@ __device__ __forceinline__ K1Rec k1_record(int64_t it, int64_t r0, int T, const 
 // HITS: the hit-list form (K1Hits) instead of the dense counts.  ISUM: with intensity sums.
 //
 // What bounds it: reading the tiles takes 0.45 of the time at 20,000 spectra on 5.7M rows (0.176 of 0.386 ms with no
-// item worked on: 0.98 GB, at 85% of the copy rate); the rest is issue and the latency of each warp's steps (0.45
+// item worked on: 0.77 GB, at 67% of the copy rate); the rest is issue and the latency of each warp's steps (0.45
 // instructions a cycle, 8 CTAs per SM), of which the exact searches take 0.13 ms, the filter 0.055, clearing and
 // writing the histograms 0.03.  Against the form before -- filter words loaded when needed, a second path for windows
 // that straddle a bitmap word, a search per coarse bin, run-time intensity branches -- a launch took, before -> now:

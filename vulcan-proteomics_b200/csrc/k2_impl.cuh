@@ -242,20 +242,23 @@ __device__ __forceinline__ K2Val k2_score(const SmemFrag& fp, const PT& pt, int 
 //   * lookup: the listed ions of all the warp's candidates, 32 at a time with every lane busy: tolerance window, first
 //     peak by a table of start indices, most intense peak, its ppm term; then every lane adds its own ions' results,
 //     b then y in ion order.  The arithmetic is k2_score's, so the outputs are bit-identical to it.
-// Residues come four at a time from aligned words (single bytes where a word would leave the row), their masses
+// Residues come four at a time from aligned words (single bytes at the ends of the table), their masses
 // from one table of mono + delta, lnfact of small counts from a table built by the same function.  A
 // candidate of more than KD_MAXLEN residues, or with more marked ions than its lists hold, is scored by k2_score;
 // with fragment charges above 1 each lane looks its own ions up, charge by charge.
 //
-// What bounds it: instruction issue and the latency of a warp's dependent steps (the walk's shared-memory tests, the
-// lookup's search and division); HBM is at 5%.  The warp-per-spectrum kernel with a lookup per ion before it ran
-// 4,700 instructions per 32 candidates at 20.7 active lanes; this one runs 2,000 at 25.2.  Measured (device time per
-// launch, before -> now): 5.92M candidates of 40,000 spectra 1.590 -> 0.708 ms, 10,001 spectra of up to 1,000
-// candidates at 20 ppm 1.412 -> 0.37, fragment charges up to 3 1.078 -> 0.337, 32 spectra 0.030 -> 0.0105.
+// What bounds it: instruction issue and the latency of a warp's dependent steps (0.6 instructions a cycle; HBM is at
+// 5%).  Of 0.341 ms for 20,000 spectra (3.0M candidates) the tables take 0.09 when nothing hides them, the walk 0.13,
+// the lookup 0.08, the hyperscore and the outputs 0.04.  The warp-per-spectrum kernel with a lookup per ion before it
+// ran 4,700 instructions per 32 candidates at 20.7 active lanes; this one runs 1,900 at 25.  Measured (device time per
+// launch, before -> now): 5.92M candidates of 40,000 spectra 1.590 -> 0.645 ms, 10,001 spectra of up to 1,000
+// candidates at 20 ppm 1.412 -> 0.324, fragment charges up to 3 1.078 -> 0.308, 32 spectra 0.030 -> 0.0096.
 // 3 warps per CTA at 8 CTAs per SM: 2, 4 and 6 warps took 12-16% longer on the 40,000 spectra (a spectrum's 148
 // candidates are 4.6 warps' worth; wider CTAs idle in their second round, narrower ones build the table with fewer).
+// Testing an ion's charges right after its mass, instead of four ions at a time, cost the overlap of the tests (0.70
+// and 0.36 ms); words that stop at each row's own end, with single bytes after them, 0.70.
 constexpr int KD_WARPS = 3;
-constexpr int KD_CTAS = 8;           // CTAs per SM (79 registers, 28 KB)
+constexpr int KD_CTAS = 8;           // CTAs per SM (80 registers, 27 KB)
 constexpr int KD_LIST = 20;          // list slots per lane and kind (a group of four ions starts with four free)
 constexpr int KD_BITS = 8192;        // presence buckets
 constexpr float KD_SCALE = 4.0f;     // buckets per Th: 2,048 Th before they wrap
@@ -283,7 +286,9 @@ __device__ __forceinline__ uint32_t kd_bucket(float m) {
 }
 __device__ __forceinline__ uint32_t kd_flag(const uint32_t* bits, float m) {
   const uint32_t q = kd_bucket(m);
-  return __funnelshift_r(bits[(q >> 5) & (KD_BITS / 32 - 1)], 0u, q) & 1u;   // shift by q mod 32
+  const uint32_t word = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(bits) +
+                                                           ((q >> 3) & (KD_BITS / 8 - 4)));   // bits[(q >> 5) % words]
+  return __funnelshift_r(word, 0u, q) & 1u;   // shift by q mod 32
 }
 
 // Ion masses that may have peak x in their tolerance window: [lo, hi] widened by 1e-6 of the masses, above the
@@ -297,35 +302,39 @@ __device__ __forceinline__ float2 kd_reach(float x, float tol_lo, float tol_hi, 
   return make_float2(__fdividef(x, up) - 2e-6f * x, __fdividef(x, dn) + 2e-6f * x);
 }
 
-// Residues of a row, four per word, from aligned words of the table that hold no byte past the row (the first may
-// begin before it).
+// Residues of a row, four per word, from aligned words of the residue table.  Words up to `end` -- the end of any row,
+// so inside the table -- are read whole, whatever row their bytes belong to; past it (the row whose end that is) and
+// before the table's first byte, only the row's own bytes are.
 struct RowWords {
-  const uint8_t* first;   // the table's first byte
-  const uint8_t* row;
+  const uint8_t* at;      // the next word
   const uint8_t* end;
-  const uint8_t* at;
-  uint32_t cur;
+  uint32_t cur, shift;
+  int left;               // bytes of the row from `at` on
 
-  __device__ __forceinline__ uint32_t fetch(const uint8_t* a) const {
-    if (a >= first && a + 4 <= end) return __ldg(reinterpret_cast<const uint32_t*>(a));
+  static __device__ __forceinline__ uint32_t bytes(const uint8_t* a, int from, int to) {
     uint32_t v = 0u;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (a + j >= row && a + j < end) v |= (uint32_t)__ldg(a + j) << (8 * j);
+      if (j >= from && j < to) v |= (uint32_t)__ldg(a + j) << (8 * j);
     return v;
   }
-  __device__ __forceinline__ void begin(const uint8_t* table, const uint8_t* r, int len) {
-    first = table;
-    row = r;
-    end = r + len;
-    at = r - (reinterpret_cast<uintptr_t>(r) & 3);
-    cur = fetch(at);
-  }
-  __device__ __forceinline__ uint32_t next() {   // the next four residues (0 past the row)
+  __device__ __forceinline__ void begin(const uint8_t* table, const uint8_t* row, int len, const uint8_t* last_end) {
+    const int skip = (int)(reinterpret_cast<uintptr_t>(row) & 3);
+    at = row - skip;
+    end = last_end;
+    shift = 8u * (uint32_t)skip;
+    left = len + skip;
+    cur = at >= table && at + 4 <= end ? __ldg(reinterpret_cast<const uint32_t*>(at)) : bytes(at, skip, left);
     at += 4;
-    const uint32_t nx = at < end ? fetch(at) : 0u;
-    const uint32_t r = __funnelshift_r(cur, nx, (uint32_t)(reinterpret_cast<uintptr_t>(row) & 3) * 8u);
+    left -= 4;
+  }
+  __device__ __forceinline__ uint32_t next() {   // the next four bytes: residues of the row, then whatever follows
+    uint32_t nx = 0u;
+    if (left > 0) nx = at + 4 <= end ? __ldg(reinterpret_cast<const uint32_t*>(at)) : bytes(at, 0, left);
+    const uint32_t r = __funnelshift_r(cur, nx, shift);
     cur = nx;
+    at += 4;
+    left -= 4;
     return r;
   }
 };
@@ -386,8 +395,82 @@ __device__ __forceinline__ double kd_lnfact(const K2DenseSmem& S, int n) {
 // Longest run of consecutive matched ion indices (run_matched: ion 0 starts no run).
 __device__ __forceinline__ int kd_longest(uint64_t hit) {
   int n = 0;
-  for (uint64_t x = hit & ~1ull; x; x &= x << 1) ++n;
+  if ((hit >> 32) == 0ull) {
+    for (uint32_t x = (uint32_t)hit & ~1u; x; x &= x << 1) ++n;
+  } else {
+    for (uint64_t x = hit & ~1ull; x; x &= x << 1) ++n;
+  }
   return n;
+}
+
+// The walk over the warp's candidates (see above): marks and lists the ions of n_max steps that may match at a charge
+// below maxfz (at most z_max in the warp).  Sets `over` where a list may have overflowed.
+__device__ __forceinline__ void kd_walk(K2DenseSmem& S, int warp, int lane, int n_ion, int n_max, int maxfz, int z_max,
+                                        RowWords& w, uint64_t mask, float b, float y, uint64_t& mark_b,
+                                        uint64_t& mark_y, bool& over) {
+  uint32_t mod_lo = (uint32_t)mask, mod_hi = (uint32_t)(mask >> 32);
+  uint32_t mb = 0u, my = 0u, mb_lo = 0u, my_lo = 0u;   // marks of the current 32 ions, of the 32 before them
+  float* list_b = &S.ion[warp][0][0][lane];
+  float* list_y = &S.ion[warp][1][0][lane];
+  for (int k0 = 0; k0 < n_max; k0 += 4) {
+    const bool in = k0 < n_ion;
+    if (k0 > KD_LIST - 4) {   // (k0 ions fill at most k0 slots) the group needs four free ones
+      if (k0 == 32) {
+        mb_lo = mb;
+        my_lo = my;
+        mb = my = 0u;
+      }
+      const int n_b = __popc(mb) + __popc(mb_lo), n_y = __popc(my) + __popc(my_lo);
+      over |= in && max(n_b, n_y) > KD_LIST - 4;
+      list_b = &S.ion[warp][0][min(n_b, KD_LIST - 4)][lane];
+      list_y = &S.ion[warp][1][min(n_y, KD_LIST - 4)][lane];
+    }
+    // byte offsets into the residue table, one per residue; past the row's end whatever follows: those ions land
+    // behind the lists' valid part and their marks are cleared by the caller
+    const uint32_t four = ((in ? w.next() : 0u) & 0x1f1f1f1fu) << 2 |
+                          (((mod_lo & 15u) * 0x00204081u) & 0x01010101u) << 7;
+    mod_lo = __funnelshift_r(mod_lo, mod_hi, 4);
+    mod_hi >>= 4;
+    float bv[4], yv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float rm = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(S.res) +
+                                                       ((four >> (8 * j)) & 0xffu));
+      bv[j] = b = __fadd_rn(b, rm);
+      yv[j] = y = __fsub_rn(y, rm);
+    }
+    uint32_t fb[4], fy[4];   // eight independent tests in flight
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      fb[j] = kd_flag(S.bits, bv[j]);
+      fy[j] = kd_flag(S.bits, yv[j]);
+    }
+    for (int z = 2; z < z_max; ++z) {
+      const uint32_t on = z < maxfz;
+      const float rz = __fdividef(1.f, (float)z);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        fb[j] |= on & kd_flag(S.bits, __fmul_rn(bv[j], rz));
+        fy[j] |= on & kd_flag(S.bits, __fmul_rn(yv[j], rz));
+      }
+    }
+    uint32_t pb = 0u, py = 0u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (in) {        // kept only when the slot moves on
+        *list_b = bv[j];
+        *list_y = yv[j];
+      }
+      list_b += fb[j] * 32u;
+      list_y += fy[j] * 32u;
+      pb += fb[j] << j;
+      py += fy[j] << j;
+    }
+    mb |= pb << (k0 & 31);
+    my |= py << (k0 & 31);
+  }
+  mark_b = n_max > 32 ? (uint64_t)mb << 32 | mb_lo : mb;
+  mark_y = n_max > 32 ? (uint64_t)my << 32 | my_lo : my;
 }
 
 // A candidate's row, loaded ahead of its scoring.
@@ -413,6 +496,16 @@ __device__ __forceinline__ DenseRow kd_row(int64_t c, const int32_t* c_row, cons
   return d;
 }
 
+// The row's first word.  Words up to the row end of the warp's last live lane are read whole (candidates come in row
+// order, so that is nearly all of them).
+__device__ __forceinline__ void kd_begin(RowWords& w, const DenseRow& d, bool live, const uint8_t* res) {
+  const unsigned lanes = __ballot_sync(VK_FULL, live);
+  if (!lanes) return;
+  const unsigned long long mine = reinterpret_cast<unsigned long long>(d.seq + d.len);
+  const unsigned long long last = __shfl_sync(VK_FULL, mine, 31 - __clz(lanes));
+  if (live && d.ions() > 0) w.begin(res, d.seq, d.len, reinterpret_cast<const uint8_t*>(last));
+}
+
 // Scores the warp's candidates (lanes with `live` hold one each).
 __device__ __forceinline__ void kd_score(K2DenseSmem& S, const DensePeaks& pt, int warp, int lane, bool live,
                                          const DenseRow& d, RowWords& w, const SmemFrag& fp, const int64_t* seq_off,
@@ -423,49 +516,10 @@ __device__ __forceinline__ void kd_score(K2DenseSmem& S, const DensePeaks& pt, i
   const int n_ion = live ? d.ions() : 0;
   const int n_max = __reduce_max_sync(VK_FULL, n_ion);
   const int z_max = __reduce_max_sync(VK_FULL, fits ? d.maxfz : 0);
-  uint64_t mark_b = 0ull, mark_y = 0ull;   // ions that may match
+  uint64_t mark_b, mark_y;   // ions that may match
   bool over = false;
-  {
-    const float nt = nterm_of(fp, d.mask);
-    float b = nt, y = __fsub_rn(d.mass, nt);
-    int n_b = 0, n_y = 0;
-    for (int k0 = 0; k0 < n_max; k0 += 4) {
-      // a residue's table index per byte; past the row's end the index is 0, whose mass is 0: those ions land behind
-      // the list's valid part and their marks are cleared below
-      const bool in = k0 < n_ion;
-      uint32_t four = in ? w.next() & 0x1f1f1f1fu : 0u;
-      const uint32_t nib = (uint32_t)(d.mask >> k0) & 15u;
-      four |= ((nib * 0x00204081u) & 0x01010101u) << 5;
-      over |= in && max(n_b, n_y) > KD_LIST - 4;
-      float* list_b = &S.ion[warp][0][min(n_b, KD_LIST - 4)][lane];
-      float* list_y = &S.ion[warp][1][min(n_y, KD_LIST - 4)][lane];
-      uint32_t pb = 0u, py = 0u;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float rm = S.res[(four >> (8 * j)) & 63u];
-        b = __fadd_rn(b, rm);
-        y = __fsub_rn(y, rm);
-        uint32_t fb = kd_flag(S.bits, b), fy = kd_flag(S.bits, y);
-        for (int z = 2; z < z_max; ++z) {
-          const uint32_t on = z < d.maxfz;
-          fb |= on & kd_flag(S.bits, __fdividef(b, (float)z));
-          fy |= on & kd_flag(S.bits, __fdividef(y, (float)z));
-        }
-        if (in) {        // kept only when the slot moves on
-          *list_b = b;
-          *list_y = y;
-        }
-        list_b += fb * 32u;
-        list_y += fy * 32u;
-        pb += fb << j;
-        py += fy << j;
-      }
-      n_b += __popc(pb);
-      n_y += __popc(py);
-      mark_b |= (uint64_t)pb << k0;
-      mark_y |= (uint64_t)py << k0;
-    }
-  }
+  const float nt = nterm_of(fp, d.mask), y0 = __fsub_rn(d.mass, nt);
+  kd_walk(S, warp, lane, n_ion, n_max, d.maxfz, z_max, w, d.mask, nt, y0, mark_b, mark_y, over);
   const uint64_t valid = n_ion < 64 ? (1ull << n_ion) - 1ull : ~0ull;
   mark_b &= valid;
   mark_y &= valid;
@@ -610,18 +664,16 @@ __device__ __forceinline__ void k2_dense_body(K2DenseSmem& S, const SmemFrag& fp
     }
     const int blast = np > 0 ? kd_start(last, pt.q0) : -1;
     for (int q = blast + 1 + tid; q < K2_BUCKETS; q += NT) S.start[q] = (uint16_t)max(np, 0);
-    RowWords w;
-    w.cur = 0u;
-    if (some && d.ions() > 0) w.begin(res, d.seq, d.len);
+    RowWords w{};
+    kd_begin(w, d, some, res);
     __syncthreads();
     for (int64_t cw = c0 + warp * 32; cw < c1; cw += NT) {   // uniform over the warp
       const int64_t c = cw + lane;
       kd_score(S, pt, warp, lane, c < c1, d, w, fp, seq_off, len, mask, mass32, res, tol_lo, tol_hi, out, c);
-      if (c + NT < c1) {
-        d = kd_row(c + NT, c_row, c_maxfz, seq_off, len, mask, mass32, res);
-        if (d.ions() > 0) w.begin(res, d.seq, d.len);
-      }
       __syncwarp();
+      const bool more = c + NT < c1;
+      if (more) d = kd_row(c + NT, c_row, c_maxfz, seq_off, len, mask, mass32, res);
+      kd_begin(w, d, more, res);
     }
   }
 }
