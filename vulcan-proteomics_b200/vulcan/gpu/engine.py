@@ -1365,13 +1365,33 @@ def _run_column(run: str, n: int) -> pa.Array:
     return col.slice(0, n)
 
 
+_ARROW_TYPES: dict = {}
+
+
+def _arrow(a: np.ndarray) -> pa.Array:
+    """The Arrow array of a 1-D numeric numpy array, on its memory.  Built from the buffer itself: pa.array looks at
+    every call for what the array might hold (3 us a column, 1.3 this way)."""
+    t = _ARROW_TYPES.get(a.dtype)
+    if t is None:
+        t = _ARROW_TYPES[a.dtype] = pa.from_numpy_dtype(a.dtype)
+    if a.ndim != 1 or not a.flags.c_contiguous or a.dtype.kind not in "iuf" or not a.dtype.isnative:
+        return pa.array(a)
+    return pa.Array.from_buffers(t, len(a), [None, pa.py_buffer(a)])
+
+
+_TABLE_NAMES = None
+
+
 def _table(sp: Spectra, rec: dict) -> pa.Table:
     """The PSM table from device-computed columns: run, scan and retention time added on the host."""
+    global _TABLE_NAMES
+    if _TABLE_NAMES is None:
+        _TABLE_NAMES = ["run", "spec_idx", "scan", "rt"] + list(_PSM_TABLE[1:])
     s = rec["spec_idx"]
-    cols = {"run": _run_column(sp.run, len(s)), "spec_idx": s, "scan": sp.scan[s], "rt": sp.rt[s]}
-    for k in _PSM_TABLE[1:]:
-        cols[k] = rec[k]
-    return pa.table(cols)
+    cols = [_run_column(sp.run, len(s)), _arrow(s), _arrow(np.asarray(sp.scan).take(s)),
+            _arrow(np.asarray(sp.rt).take(s))]
+    cols += [_arrow(rec[k]) for k in _PSM_TABLE[1:]]
+    return pa.Table.from_arrays(cols, names=_TABLE_NAMES)
 
 
 def _read_packed(buf: torch.Tensor, layout, sp: Spectra, stats: Stats | None = None) -> pa.Table:
@@ -1408,11 +1428,13 @@ def _pinned_like(a: np.ndarray) -> np.ndarray:
                        pin_memory=True).numpy()
 
 
-def _is_pinned(a: np.ndarray) -> bool:
+def _pinned_view(a: np.ndarray):
+    """a as a tensor when its memory is pinned, else None."""
     try:
-        return bool(torch.from_numpy(a).is_pinned())
+        t = torch.from_numpy(a)
+        return t if t.is_pinned() else None
     except (TypeError, ValueError, RuntimeError):
-        return False
+        return None
 
 
 class _ResultPool:
@@ -1464,6 +1486,7 @@ class _Slot:
         # the packed PSMs' landing buffer when the shape's result pool has none free: read into copies at once
         self.host_out = torch.empty(self.out_bytes, dtype=torch.uint8, pin_memory=True)
         self.offsets = torch.empty(n + 1, dtype=torch.int64, pin_memory=True)   # offsets staging
+        self.status = torch.zeros(1, dtype=torch.int32, pin_memory=True)         # the pass's status, read back with it
         self.stage = {}
         self.h2d_done = torch.cuda.Event()
         self.done = torch.cuda.Event()
@@ -1528,8 +1551,9 @@ class Searcher:
     def _shape(self, parts, n_total: int):
         """(spectra, peak capacity, largest peak count, hypothesis capacity) of consecutive runs padded to n_total
         spectra (padding: empty spectra of known charge)."""
-        n_raw = sum(int(np.asarray(sp.offsets)[-1]) for sp in parts)
-        mr = max((int(np.diff(np.asarray(sp.offsets, np.int64)).max()) for sp in parts if len(sp)), default=0)
+        offs = [np.asarray(sp.offsets, np.int64) for sp in parts]
+        n_raw = sum(int(o[-1]) for o in offs)
+        mr = max((int((o[1:] - o[:-1]).max()) for o in offs if len(o) > 1), default=0)
         z0, z1 = self.p.precursor_charge
         i0, i1 = self.p.isotope_errors
         n_max = sum(self._n_hyp(sp) for sp in parts) + (n_total - sum(len(sp) for sp in parts)) * (i1 - i0 + 1)
@@ -1566,50 +1590,56 @@ class Searcher:
                 base_pk += int(o[-1])
                 base_sp += len(sp)
             offs[base_sp + 1:] = base_pk
-            # the previous pass over this slot and its read-back must be done before its buffers are reused
-            self.copy_stream.wait_event(slot.done)
-            h2d = 0
-            with torch.cuda.stream(self.copy_stream):
+            # the streams are set one after another and the caller's restored at the end (a stream context costs 12 us)
+            caller = torch.cuda.current_stream(self.gi.dev)
+            try:
+                # the previous pass over this slot and its read-back must be done before its buffers are reused
+                torch.cuda.set_stream(self.copy_stream)
+                self.copy_stream.wait_event(slot.done)
                 run.offsets.copy_(slot.offsets, non_blocking=True)
-                h2d += slot.offsets.numel() * 8
+                h2d = slot.offsets.numel() * 8
                 bp = bs = 0
                 for j, sp in enumerate(parts):
-                    nr = int(np.asarray(sp.offsets)[-1])
+                    nr = int(sp.offsets[-1])
                     ns = len(sp)
-                    for name, dst, a, lo, cnt in (("mz", run.mz, sp.mz, bp, nr), ("int", run.intensity, sp.intensity, bp, nr),
-                                                  ("pmz", run.precursor_mz, sp.precursor_mz, bs, ns),
-                                                  ("z", run.charge, sp.charge, bs, ns)):
+                    for name, dst, a, lo, cnt, dt in (("mz", run.mz, sp.mz, bp, nr, np.float32),
+                                                      ("int", run.intensity, sp.intensity, bp, nr, np.float32),
+                                                      ("pmz", run.precursor_mz, sp.precursor_mz, bs, ns, np.float64),
+                                                      ("z", run.charge, sp.charge, bs, ns, np.int8)):
                         if cnt == 0:
                             continue
-                        dt = torch.empty(0, dtype=dst.dtype).numpy().dtype
                         a = np.asarray(a)[:cnt]
-                        if a.dtype != dt or not a.flags.c_contiguous or not _is_pinned(a):
-                            a = slot.staged((name, j), np.ascontiguousarray(a, dtype=dt))
-                        dst[lo:lo + cnt].copy_(torch.from_numpy(a), non_blocking=True)
-                        h2d += a.nbytes
+                        t = _pinned_view(a) if a.dtype == dt and a.flags.c_contiguous else None
+                        if t is None:
+                            t = torch.from_numpy(slot.staged((name, j), np.ascontiguousarray(a, dtype=dt)))
+                        (dst if cnt == dst.numel() else dst[lo:lo + cnt]).copy_(t, non_blocking=True)
+                        h2d += cnt * t.element_size()
                     bp += nr
                     bs += ns
                 if bs < n_total:
                     run.precursor_mz[bs:n_total].fill_(0.0)
                     run.charge[bs:n_total].fill_(1)
-            slot.h2d_done.record(self.copy_stream)
-            self.compute_stream.wait_event(slot.h2d_done)
-            ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
-            with torch.cuda.stream(self.compute_stream):
+                slot.h2d_done.record(self.copy_stream)
+                self.compute_stream.wait_event(slot.h2d_done)
+                ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+                torch.cuda.set_stream(self.compute_stream)
                 ev[0].record(self.compute_stream)
                 out = slot.gp.replay()
                 ev[1].record(self.compute_stream)
-            self.d2h_stream.wait_event(ev[1])
-            pool = self.pools.get(slot.out_bytes)
-            if pool is None:
-                pool = self.pools[slot.out_bytes] = _ResultPool(slot.out_bytes, self.hold_bytes // slot.out_bytes)
-            host_out = pool.take()
-            lent = host_out is not None
-            if not lent:
-                host_out = slot.host_out
-            with torch.cuda.stream(self.d2h_stream):
+                self.d2h_stream.wait_event(ev[1])
+                pool = self.pools.get(slot.out_bytes)
+                if pool is None:
+                    pool = self.pools[slot.out_bytes] = _ResultPool(slot.out_bytes, self.hold_bytes // slot.out_bytes)
+                host_out = pool.take()
+                lent = host_out is not None
+                if not lent:
+                    host_out = slot.host_out
+                torch.cuda.set_stream(self.d2h_stream)
                 host_out.copy_(out["packed"], non_blocking=True)
+                slot.status.copy_(out["status"], non_blocking=True)
                 slot.done.record(self.d2h_stream)
+            finally:
+                torch.cuda.set_stream(caller)
             return (parts[0] if len(parts) == 1 else None, slot, h2d, ev, host_out, pool if lent else None)
 
     def held_bytes(self) -> int:
@@ -1622,7 +1652,7 @@ class Searcher:
         slot.done.synchronize()
         t1 = time.perf_counter()
         self.device_ms += ev[0].elapsed_time(ev[1])
-        check_status(slot.gp.out["status"])
+        check_status(slot.status)
         nb = host_out.numel()
         host = host_out.numpy()
         rec = _unpack_psms(host, slot.layout, copy=pool is None)
