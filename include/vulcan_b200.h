@@ -554,6 +554,22 @@ int vk_bce(int n, const float* z, const float* y, const float* w, float inv_wsum
  * given */
 int vk_adam(int64_t n, float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
             int step, float wd, void* p_bf16, void* stream);
+/* The same step on up to VK_ADAM_MAX tensors in one launch. */
+#define VK_ADAM_MAX 8
+typedef struct {
+  int64_t n;        /* elements */
+  float* p;         /* FP32 master weights */
+  const float* g;   /* gradient */
+  float* m;         /* first and second moments */
+  float* v;
+  void* p_bf16;     /* BF16 copy, or NULL */
+} vk_adam_tensor;
+int vk_adam_group(const vk_adam_tensor* t, int n_tensors, float lr, float b1, float b2, float eps, int step, float wd,
+                  void* stream);
+/* A mini-batch of n training rows: Xb[i] = X[idx[i]] (width floats a row), yb[i] = y[idx[i]], wb[i] = w[idx[i]];
+ * 0 <= idx[i] < the rows of X */
+int vk_gather_batch(const int64_t* idx, int n, const float* X, int width, const float* y, const float* w, float* Xb,
+                    float* yb, float* wb, void* stream);
 int vk_to_bf16(int64_t n, const float* x, void* y, void* stream);
 int vk_bf16_to_f32(int64_t n, const void* x, float* y, void* stream);
 

@@ -78,3 +78,42 @@ def test_layer3_gemm_equals_sequential_sums(M, N, K, sam, scm, b_bf16, bias, rel
                               rnd, KL.ptr(C), scm, 1, KL.stream()), "gemm")
     assert torch.equal(C[:, :N].cpu(), want)
     assert bool((C[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("sizes", [(1,), (256, 1, 4096), (65536, 256, 65536, 256, 256, 1), (5, 7, 300, 1, 2, 3, 4, 6)])
+def test_adam_group_equals_adam(sizes):
+    import ctypes as C
+
+    import torch
+    from vulcan.gpu import _lib as KL
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    rnd = lambda n: torch.randn(n, device="cuda", generator=g)  # noqa: E731
+    one = [[rnd(n), rnd(n), rnd(n) * 0.1, rnd(n).abs() * 0.01, torch.zeros(n, dtype=torch.bfloat16, device="cuda")]
+           for n in sizes]
+    two = [[x.clone() for x in t] for t in one]
+    for step in (1, 2, 9):
+        arr = (KL.AdamTensor * len(sizes))()
+        for s, (p, gr, m, v, bf), k in zip(arr, two, range(len(sizes))):
+            s.n, s.p, s.g, s.m, s.v = p.numel(), KL.ptr(p), KL.ptr(gr), KL.ptr(m), KL.ptr(v)
+            s.p_bf16 = KL.ptr(bf) if k % 2 else None
+        KL.check(KL.lib().vk_adam_group(C.byref(arr), len(sizes), 2e-3, 0.9, 0.999, 1e-8, step, 0.01, KL.stream()),
+                 "adam")
+        for k, (p, gr, m, v, bf) in enumerate(one):
+            KL.check(KL.lib().vk_adam(p.numel(), KL.ptr(p), KL.ptr(gr), KL.ptr(m), KL.ptr(v), 2e-3, 0.9, 0.999, 1e-8,
+                                      step, 0.01, KL.ptr(bf) if k % 2 else None, KL.stream()), "adam")
+    for a, b in zip(one, two):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("n,rows,width,off", [(1, 1, 16, 0), (1000, 333, 16, 0), (257, 5000, 16, 1), (64, 90, 6, 0)])
+def test_gather_batch_equals_indexing(n, rows, width, off):
+    import torch
+    from vulcan.gpu import _lib as KL
+    X = torch.randn(rows * width + off, device="cuda")[off:].view(rows, width)
+    y, w = torch.randn(rows, device="cuda"), torch.randn(rows, device="cuda")
+    idx = torch.randint(rows, (n,), device="cuda")
+    out = [torch.zeros(n, width, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")]
+    KL.check(KL.lib().vk_gather_batch(KL.ptr(idx), n, KL.ptr(X), width, KL.ptr(y), KL.ptr(w),
+                                      *[KL.ptr(t) for t in out], KL.stream()), "gather_batch")
+    for got, src in zip(out, (X, y, w)):
+        assert torch.equal(got, src[idx])

@@ -64,6 +64,11 @@ class CandOut(C.Structure):
     _fields_ = [("cap", C.c_int), ("n_cand", P), ("c_hyp", P), ("c_row", P), ("c_cnt", P)] + _K2_FIELDS
 
 
+class AdamTensor(C.Structure):
+    """vk_adam_tensor"""
+    _fields_ = [("n", I64), ("p", P), ("g", P), ("m", P), ("v", P), ("p_bf16", P)]
+
+
 # reference-compatible signatures (vulcan/gpu/_lib.py:22-35 of the reference)
 _SIGS = {
     "vk_set_params": [P, P, P],
@@ -122,6 +127,8 @@ _SIGS_B200 = {
     "vk_relu_mask": [I64, P, P, P],
     "vk_bce": [I32, P, P, P, F32, P, P, P],
     "vk_adam": [I64, P, P, P, P, F32, F32, F32, F32, I32, F32, P, P],
+    "vk_adam_group": [P, I32, F32, F32, F32, F32, I32, F32, P],
+    "vk_gather_batch": [P, I32, P, I32, P, P, P, P, P, P],
     "vk_to_bf16": [I64, P, P, P],
     "vk_bf16_to_f32": [I64, P, P, P],
 }

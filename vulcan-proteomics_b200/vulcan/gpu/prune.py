@@ -227,14 +227,20 @@ class Pruner:
         self._colsum(B, HIDDEN, bf["dH1"], None, g["b1"], "colsum_b1")
         return bf["loss"][:(B + 255) // 256], g
 
-    def adam_step(self, lr: float, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, wd: float = 0.0):
-        L = K.lib()
-        self.step += 1
-        for k in _PARAMS:
+    def _adam_group(self):
+        """The tensors of an Adam step as vk_adam_group takes them."""
+        t = (K.AdamTensor * len(_PARAMS))()
+        for s, k in zip(t, _PARAMS):
             m, v = self._adam[k]
-            K.check(L.vk_adam(self.w[k].numel(), K.ptr(self.w[k]), K.ptr(self._grad[k]), K.ptr(m), K.ptr(v), lr,
-                              b1, b2, eps, self.step, wd, K.ptr(self.bf[k]) if k in self.bf else None, K.stream()),
-                    "adam")
+            s.n, s.p, s.g, s.m, s.v = (self.w[k].numel(), K.ptr(self.w[k]), K.ptr(self._grad[k]), K.ptr(m), K.ptr(v))
+            s.p_bf16 = K.ptr(self.bf.get(k))
+        return t
+
+    def adam_step(self, lr: float, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, wd: float = 0.0, group=None):
+        """One Adam step on every parameter.  group: ``_adam_group()`` of the current tensors (fit builds it once)."""
+        self.step += 1
+        t = self._adam_group() if group is None else group
+        K.check(K.lib().vk_adam_group(C.byref(t), len(_PARAMS), lr, b1, b2, eps, self.step, wd, K.stream()), "adam")
 
     def set_standardisation(self, raw_feat: torch.Tensor):
         x = raw_feat[:, :N_FEAT].float()
@@ -255,6 +261,10 @@ class Pruner:
         wt = (torch.ones(n, device=self.dev) if weight is None else weight.to(self.dev, torch.float32)).contiguous()
         g = torch.Generator(device=self.dev).manual_seed(seed)
         B = min(batch, n)
+        Xb = torch.empty(B, N_IN, dtype=torch.float32, device=self.dev)
+        yb, wb = (torch.empty(B, dtype=torch.float32, device=self.dev) for _ in range(2))
+        self._buffers(B)
+        group = self._adam_group()
         losses = []
         n_batch = n // B
         for ep in range(epochs):
@@ -264,11 +274,12 @@ class Pruner:
             # cosine learning-rate decay over all steps
             for i in range(n_batch):
                 idx = perm[i * B:(i + 1) * B]
-                Xb, yb, wb = X[idx].contiguous(), y[idx].contiguous(), wt[idx].contiguous()
+                K.check(L.vk_gather_batch(K.ptr(idx), B, K.ptr(X), N_IN, K.ptr(y), K.ptr(wt), K.ptr(Xb), K.ptr(yb),
+                                          K.ptr(wb), K.stream()), "gather_batch")
                 self.forward_train(Xb, B)
                 loss, _ = self.backward(Xb, yb, wb, B, 1.0 / B)
                 frac = (ep * n_batch + i) / max(1, epochs * n_batch)
-                self.adam_step(lr * 0.5 * (1.0 + math.cos(math.pi * frac)), wd=wd)
+                self.adam_step(lr * 0.5 * (1.0 + math.cos(math.pi * frac)), wd=wd, group=group)
                 tot += loss.sum()
             losses.append(float(tot) / max(n_batch, 1))
             E.check_status(self._buf["status"], "training GEMM")
