@@ -120,6 +120,11 @@ __device__ __forceinline__ uint64_t smem_kth_largest_radix(const uint64_t* key, 
   return prefix;
 }
 
+// Spectra a warp of the launch over the left ones looks at.  A left spectrum keeps its warp for some 50 us, so they are
+// dealt in small groups over many CTAs; 32 at a time by 296 CTAs took 0.65 ms on 40,000 spectra of an index where many
+// partners fall beside the window (masses of a pair that round differently), 8 / 4 / 2 / 1 take 0.320 / 0.286 / 0.295 /
+// 0.319; with none left 0.002 / 0.004 / 0.007 / 0.010 ms.
+constexpr int TK_REST = 4;
 #ifndef TK_UNROLL
 #define TK_UNROLL 8            // count loads in flight per lane
 #endif
@@ -535,8 +540,8 @@ select_topk_k(int n_spec, int rest, const int64_t* spec_hyp_off, const int64_t* 
     for (int s = first; s < n_spec; s += step) one(s);
     return;
   }
-  for (int s0 = first * 32; s0 < n_spec; s0 += step * 32) {
-    unsigned left = __ballot_sync(VK_FULL, s0 + lane < n_spec && n_cand[s0 + lane] < 0);
+  for (int s0 = first * TK_REST; s0 < n_spec; s0 += step * TK_REST) {
+    unsigned left = __ballot_sync(VK_FULL, lane < TK_REST && s0 + lane < n_spec && n_cand[s0 + lane] < 0);
     for (; left; left &= left - 1u) one(s0 + __ffs(left) - 1);
   }
 }
@@ -1275,9 +1280,7 @@ int vk_select_topk(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
         c_hyp, c_row, c_cnt, n_cand, hyp_scored, hyp_matched, spec_scored, spec_matched);
     const int rc = vk_launch_status();
     if (rc != 0) return rc;
-    // a few CTAs look for the spectra left over, 32 flags at a time
-    grid = (unsigned)((n_spec + TK_WARPS * 32 - 1) / (TK_WARPS * 32));
-    if (grid > 296u) grid = 296u;
+    grid = (unsigned)((n_spec + TK_WARPS * TK_REST - 1) / (TK_WARPS * TK_REST));
   }
   select_topk_k<<<grid, TK_WARPS * 32, sh, (cudaStream_t)stream>>>(
       n_spec, rest, spec_hyp_off, h_lo, h_hi, win_off, cnt, cnt_cap, partner, thr, topk, pair_closure, cap, list_pow2,
