@@ -322,8 +322,8 @@ int vk_compact_hits(int n_spec, int cap, const int64_t* n_cand, const int64_t* c
                     int64_t* c_hyp, int64_t* c_row, int64_t* c_cnt, int32_t* c_row32, int8_t* c_maxfz,
                     uint32_t* c_isum, void* stream);
 
-/* K2 exact rescoring (reference kernels.cu:263-376), B200 launch: one warp per spectrum, lanes over candidates,
- * the spectrum's (first 512) peaks in shared memory.  Candidates of spectrum s are [cand_off[s], cand_off[s+1])
+/* K2 exact rescoring (reference kernels.cu:263-376), B200 launch: a CTA per spectrum at a time (one warp with
+ * c_shift), lanes over candidates, the spectrum's (first 512) peaks in shared memory.  Candidates of spectrum s are [cand_off[s], cand_off[s+1])
  * (cand_off has n_spec+1 entries, spectrum ids are 0..n_spec-1).  c_shift NULL: the closed mode; else the
  * per-candidate precursor shift (Da, f32) of the open / mass-offset modes: shifted and unshifted ions scored as
  * the reference's shift mode (kernels.cu:294-363). */

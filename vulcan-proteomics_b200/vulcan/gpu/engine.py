@@ -989,7 +989,7 @@ def _compact(n: int, cap: int, n_cand, s_hyp, s_row, s_cnt, dh, dev):
 
 def _k2_cands(gi: GpuIndex, p: SearchParams, n: int, cand, peaks, sparse: bool = False):
     """K2 over compacted candidate lists; one output row per candidate.  Dense lists (the exhaustive path's top-k
-    per spectrum): ``vk_k2_spectra``, a warp per spectrum over its staged peaks; sparse lists (a few candidates per
+    per spectrum): ``vk_k2_spectra``, a CTA per spectrum over its staged peaks; sparse lists (a few candidates per
     spectrum after the pruner): ``vk_k2_cands``, a thread per candidate.  Same outputs."""
     L = K.lib()
     dev = gi.dev
