@@ -480,7 +480,8 @@ struct DenseRow {
   float mass;
   int row, len, maxfz;
 
-  __device__ __forceinline__ int ions() const { return len <= KD_MAXLEN && maxfz > 1 ? len - 1 : 0; }
+  // ions to walk; none of an empty row (whose offset may lie anywhere: its residues are not looked at)
+  __device__ __forceinline__ int ions() const { return len <= KD_MAXLEN && maxfz > 1 ? max(len - 1, 0) : 0; }
 };
 
 __device__ __forceinline__ DenseRow kd_row(int64_t c, const int32_t* c_row, const int8_t* c_maxfz,
@@ -496,10 +497,10 @@ __device__ __forceinline__ DenseRow kd_row(int64_t c, const int32_t* c_row, cons
   return d;
 }
 
-// The row's first word.  Words up to the row end of the warp's last live lane are read whole (candidates come in row
-// order, so that is nearly all of them).
+// The row's first word.  Words up to the row end of the warp's last lane with ions are read whole (candidates come in
+// row order, so that is nearly all of them).
 __device__ __forceinline__ void kd_begin(RowWords& w, const DenseRow& d, bool live, const uint8_t* res) {
-  const unsigned lanes = __ballot_sync(VK_FULL, live);
+  const unsigned lanes = __ballot_sync(VK_FULL, live && d.ions() > 0);
   if (!lanes) return;
   const unsigned long long mine = reinterpret_cast<unsigned long long>(d.seq + d.len);
   const unsigned long long last = __shfl_sync(VK_FULL, mine, 31 - __clz(lanes));
