@@ -236,10 +236,11 @@ class Pruner:
             s.p_bf16 = K.ptr(self.bf.get(k))
         return t
 
-    def adam_step(self, lr: float, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, wd: float = 0.0, group=None):
-        """One Adam step on every parameter.  group: ``_adam_group()`` of the current tensors (fit builds it once)."""
+    def adam_step(self, lr: float, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, wd: float = 0.0):
+        """One Adam step on every parameter.  The addresses are read at every step (10 us): what runs between two steps
+        -- a callback of fit that loads other weights, a subclass that replaces gradients -- may change the tensors."""
         self.step += 1
-        t = self._adam_group() if group is None else group
+        t = self._adam_group()
         K.check(K.lib().vk_adam_group(C.byref(t), len(_PARAMS), lr, b1, b2, eps, self.step, wd, K.stream()), "adam")
 
     def set_standardisation(self, raw_feat: torch.Tensor):
@@ -263,8 +264,6 @@ class Pruner:
         B = min(batch, n)
         Xb = torch.empty(B, N_IN, dtype=torch.float32, device=self.dev)
         yb, wb = (torch.empty(B, dtype=torch.float32, device=self.dev) for _ in range(2))
-        self._buffers(B)
-        group = self._adam_group()
         losses = []
         n_batch = n // B
         for ep in range(epochs):
@@ -279,7 +278,7 @@ class Pruner:
                 self.forward_train(Xb, B)
                 loss, _ = self.backward(Xb, yb, wb, B, 1.0 / B)
                 frac = (ep * n_batch + i) / max(1, epochs * n_batch)
-                self.adam_step(lr * 0.5 * (1.0 + math.cos(math.pi * frac)), wd=wd, group=group)
+                self.adam_step(lr * 0.5 * (1.0 + math.cos(math.pi * frac)), wd=wd)
                 tot += loss.sum()
             losses.append(float(tot) / max(n_batch, 1))
             E.check_status(self._buf["status"], "training GEMM")
