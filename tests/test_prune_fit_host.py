@@ -72,3 +72,16 @@ def test_adam_takes_gradients_replaced_between_steps(pruner):
             super().adam_step(lr, b1, b2, eps, wd)
     Clipped("cpu").fit(torch.zeros(64, PR.N_IN, dtype=torch.bfloat16), torch.zeros(64), epochs=1, batch=32)
     assert [[t[2] for t in step] for step in rec.adam] == [[g[k].data_ptr() for k in PR._PARAMS] for g in grads]
+
+
+@pytest.mark.parametrize("shape,ok", [((64,), True), ((70,), True), ((64, 1), True), ((63,), False), ((1,), False),
+                                      ((1, 64), False), ((), False)])
+def test_weights_have_a_row_per_target(pruner, shape, ok):
+    PR, pr, rec = pruner
+    args = (torch.zeros(64, PR.N_IN, dtype=torch.bfloat16), torch.zeros(64), torch.ones(shape))
+    if ok:
+        assert len(pr.fit(*args, epochs=1, batch=32)) == 1
+    else:
+        with pytest.raises(ValueError):
+            pr.fit(*args, epochs=1, batch=32)
+        assert not rec.adam

@@ -256,6 +256,9 @@ class Pruner:
         of every epoch.  Mini-batches in a seeded order; the last partial batch is dropped."""
         L = K.lib()
         n = len(y)
+        # a mini-batch is gathered by row number, with no bounds check on the device
+        if weight is not None and (weight.dim() == 0 or len(weight) < n):
+            raise ValueError(f"fit: {n} targets, weights of shape {tuple(weight.shape)}")
         X = torch.empty(n, N_IN, dtype=torch.float32, device=self.dev)
         K.check(L.vk_bf16_to_f32(n * N_IN, K.ptr(feat), K.ptr(X), K.stream()), "bf16_to_f32")
         y = y.to(self.dev, torch.float32).contiguous()
