@@ -1371,11 +1371,11 @@ _ARROW_TYPES: dict = {}
 def _arrow(a: np.ndarray) -> pa.Array:
     """The Arrow array of a 1-D numeric numpy array, on its memory.  Built from the buffer itself: pa.array looks at
     every call for what the array might hold (3 us a column, 1.3 this way)."""
+    if a.ndim != 1 or not a.flags.c_contiguous or a.dtype.kind not in "iuf" or not a.dtype.isnative:
+        return pa.array(a)
     t = _ARROW_TYPES.get(a.dtype)
     if t is None:
         t = _ARROW_TYPES[a.dtype] = pa.from_numpy_dtype(a.dtype)
-    if a.ndim != 1 or not a.flags.c_contiguous or a.dtype.kind not in "iuf" or not a.dtype.isnative:
-        return pa.array(a)
     return pa.Array.from_buffers(t, len(a), [None, pa.py_buffer(a)])
 
 
