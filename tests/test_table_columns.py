@@ -1,4 +1,5 @@
-"""The host columns of a PSM table: scan numbers and retention times of any kind that pa.array takes."""
+"""The host columns of a PSM table: scan numbers and retention times of any kind that pa.array takes; and the Searcher
+on runs whose arrays are of other array types."""
 import datetime
 
 import numpy as np
@@ -26,3 +27,20 @@ def test_table_takes_every_column_kind(scan, rt):
     assert t.column("scan").combine_chunks() == pa.array(scan[s])
     assert t.column("rt").combine_chunks() == pa.array(rt[s])
     assert t.num_rows == 3 and t.column("run").to_pylist() == ["r"] * 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["list", "series", "arrow"])
+def test_searcher_takes_offsets_of_any_array_type(mini, kind):
+    import dataclasses
+
+    import pandas as pd
+    from vulcan.gpu import engine as E
+    from vulcan.gpu.host import SearchParams
+    l1, sp, _ = mini
+    p = SearchParams(fragment_ppm=(-0.02, 0.02), fragment_unit="da", max_fragment_charge=1)
+    gi = E.GpuIndex(l1, p, {"C": 57.021464}, {"M": 15.9949})
+    off = {"list": list, "series": pd.Series, "arrow": pa.array}[kind](sp.offsets.tolist())
+    want = E.Searcher(gi, l1, p).search(sp)[0]
+    assert want.num_rows > 0
+    assert E.Searcher(gi, l1, p).search(dataclasses.replace(sp, offsets=off))[0].equals(want)

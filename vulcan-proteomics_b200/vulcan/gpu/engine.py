@@ -1600,7 +1600,7 @@ class Searcher:
                 h2d = slot.offsets.numel() * 8
                 bp = bs = 0
                 for j, sp in enumerate(parts):
-                    nr = int(sp.offsets[-1])
+                    nr = int(np.asarray(sp.offsets)[-1])
                     ns = len(sp)
                     for name, dst, a, lo, cnt, dt in (("mz", run.mz, sp.mz, bp, nr, np.float32),
                                                       ("int", run.intensity, sp.intensity, bp, nr, np.float32),
