@@ -316,7 +316,7 @@ int k1_tiles_launch(const vk_tindex* ix, const vk_frag_params* fp, float tol_lo,
   if (ISUM && (!pk_int || !tic)) return VK_E_ARG;
   const size_t sh = (size_t)ix->max_tile_postings * 4 + (size_t)stride * 2 + (size_t)nb * vk::K1_BM_WORDS * 4 +
                     (size_t)warps * (T * 4 * (ISUM ? 2 : 1) + vk::K1_QUEUE * 4);
-  if (sh > 200 * 1024) return VK_E_TOO_LARGE;
+  if (sh > 200 * 1024 + (size_t)warps * (vk::K1_QUEUE - 64) * 4) return VK_E_TOO_LARGE;   // (200 KB at queues of 64)
   cudaError_t e = cudaFuncSetAttribute(k1_tiles_k<HITS, ISUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (e != cudaSuccess) return vk_err(e);
   k1_tiles_k<HITS, ISUM><<<(unsigned)ix->n_tiles, warps * 32, sh, (cudaStream_t)stream>>>(
