@@ -168,3 +168,10 @@ __device__ __forceinline__ long long warp_sum(long long v) {
 
 static inline int vk_err(cudaError_t e) { return (int)e; }
 static inline int vk_launch_status() { return (int)cudaGetLastError(); }
+// Dynamic shared memory a kernel may be launched with.  The setting belongs to the kernel, not to a launch, and host
+// threads share it: it is always set to the most any call takes, so that no thread lowers it between another's call
+// and launch.
+template <class F>
+static inline int vk_max_smem(F kernel, size_t most) {
+  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}

@@ -316,9 +316,10 @@ int k1_tiles_launch(const vk_tindex* ix, const vk_frag_params* fp, float tol_lo,
   if (ISUM && (!pk_int || !tic)) return VK_E_ARG;
   const size_t sh = (size_t)ix->max_tile_postings * 4 + (size_t)stride * 2 + (size_t)nb * vk::K1_BM_WORDS * 4 +
                     (size_t)warps * (T * 4 * (ISUM ? 2 : 1) + vk::K1_QUEUE * 4);
-  if (sh > 200 * 1024 + (size_t)warps * (vk::K1_QUEUE - 64) * 4) return VK_E_TOO_LARGE;   // (200 KB at queues of 64)
-  cudaError_t e = cudaFuncSetAttribute(k1_tiles_k<HITS, ISUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  if (e != cudaSuccess) return vk_err(e);
+  constexpr size_t most = 200 * 1024, queue = (vk::K1_QUEUE - 64) * 4;   // 200 KB beside queues of 64
+  if (sh > most + warps * queue) return VK_E_TOO_LARGE;
+  const int rc = vk_max_smem(k1_tiles_k<HITS, ISUM>, most + K1_MAX_WARPS * queue);
+  if (rc != 0) return rc;
   k1_tiles_k<HITS, ISUM><<<(unsigned)ix->n_tiles, warps * 32, sh, (cudaStream_t)stream>>>(
       *ix, tol_lo, tol_hi, fp->tol_da, ix->max_tile_postings, tile_item_off, item_hyp, n_hyp, item_cap, h_spec,
       h_maxfz, h_lo, h_hi, win_off, cnt_cap, pk_off, pk_mass, cnt, status, pk_int, tic, isum,

@@ -38,6 +38,7 @@ constexpr int TG_SMEM_A = TG_M * TG_KC * 2;        // 32 KB
 constexpr int TG_SMEM_B = TG_N * TG_KC * 2;        // 32 KB
 constexpr int TG_BUF = TG_SMEM_A + TG_SMEM_B;
 constexpr int TG_SLACK = 128;                      // alignment of the dynamic shared memory
+constexpr size_t TG_MOST = 2 * TG_BUF + TG_SLACK;
 constexpr int TG_BATCH = 4;                        // items loaded ahead per thread
 
 __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
@@ -256,22 +257,21 @@ int vk_tc_gemm(int M, int N, int K, const float* A, int64_t sam, int64_t sak, co
   dim3 grid((unsigned)((M + TG_M - 1) / TG_M), (unsigned)((N + TG_N - 1) / TG_N), (unsigned)splits);
   const int buffers = ks > TG_KC ? 2 : 1;
   const int smem = buffers * TG_BUF + TG_SLACK;
-  cudaError_t e;
   if (b_bf16) {
-    e = cudaFuncSetAttribute(tc_gemm_k<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return vk_err(e);
+    const int rc = vk_max_smem(tc_gemm_k<__nv_bfloat16>, TG_MOST);
+    if (rc != 0) return rc;
     tc_gemm_k<__nv_bfloat16><<<grid, TG_THREADS, smem, st>>>(
         M, N, K, ks, buffers, A, sam, sak, reinterpret_cast<const __nv_bfloat16*>(B), sbk, sbn, bias, relu, round_bf16,
         C, scm, scn, ws, status);
   } else {
-    e = cudaFuncSetAttribute(tc_gemm_k<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return vk_err(e);
+    const int rc = vk_max_smem(tc_gemm_k<float>, TG_MOST);
+    if (rc != 0) return rc;
     tc_gemm_k<float><<<grid, TG_THREADS, smem, st>>>(M, N, K, ks, buffers, A, sam, sak,
                                                      reinterpret_cast<const float*>(B), sbk, sbn, bias, relu,
                                                      round_bf16, C, scm, scn, ws, status);
   }
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return vk_err(e);
+  const int rc = vk_launch_status();
+  if (rc != 0) return rc;
   if (splits > 1) {
     const int64_t n = (int64_t)M * N;
     tc_gemm_reduce_k<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(M, N, splits, ws, bias, relu, round_bf16, C, scm,

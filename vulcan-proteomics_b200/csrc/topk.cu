@@ -18,6 +18,7 @@
 namespace {
 
 constexpr int TK_WARPS = 4;
+constexpr size_t TK_SMEM = 220 * 1024;   // the most shared memory a CTA takes; longer lists are refused
 
 struct WarpLists {
   uint64_t* key;   // sort keys
@@ -1264,21 +1265,21 @@ int vk_select_topk(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   const int key_cap = list_pow2 > 512 ? list_pow2 : 512;   // sort path up to 512 appended entries
   size_t per_warp = (size_t)key_cap * 8 + (size_t)list_pow2 * 12 + 1024;
   size_t sh = per_warp * TK_WARPS;
-  if (sh > 220 * 1024) return VK_E_ARG;
-  cudaError_t e = cudaFuncSetAttribute(select_topk_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  if (e != cudaSuccess) return vk_err(e);
+  if (sh > TK_SMEM) return VK_E_ARG;
+  int rc = vk_max_smem(select_topk_k, TK_SMEM);
+  if (rc != 0) return rc;
   const unsigned blocks = (unsigned)((n_spec + TK_WARPS - 1) / TK_WARPS);
   unsigned grid = blocks;
   const int rest = topk_by_rows(thr, topk);
   if (rest) {
     const int list_len = ((topk > 256 ? topk : 256) + 3) & ~3;   // each warp's scratch on a 16-byte boundary
     const size_t rsh = (sizeof(RowsScratch) + (size_t)list_len * 4) * TK_WARPS;
-    e = cudaFuncSetAttribute(select_topk_rows_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsh);
-    if (e != cudaSuccess) return vk_err(e);
+    rc = vk_max_smem(select_topk_rows_k, (sizeof(RowsScratch) + (size_t)TR_TOPK * 4) * TK_WARPS);
+    if (rc != 0) return rc;
     select_topk_rows_k<<<blocks, TK_WARPS * 32, rsh, (cudaStream_t)stream>>>(
         n_spec, spec_hyp_off, h_lo, h_hi, win_off, cnt, cnt_cap, partner, thr, topk, pair_closure, cap, list_len,
         c_hyp, c_row, c_cnt, n_cand, hyp_scored, hyp_matched, spec_scored, spec_matched);
-    const int rc = vk_launch_status();
+    rc = vk_launch_status();
     if (rc != 0) return rc;
     grid = (unsigned)((n_spec + TK_WARPS * TK_REST - 1) / (TK_WARPS * TK_REST));
   }
@@ -1331,19 +1332,19 @@ int vk_select_hits(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   const int key_cap = list_pow2 > 512 ? list_pow2 : 512;
   const size_t per_warp = (size_t)key_cap * 12 + (size_t)list_pow2 * 16 + 1024 + sizeof(HitScratch);
   const size_t sh = per_warp * TK_WARPS;
-  if (sh > 220 * 1024) return VK_E_ARG;
-  cudaError_t e = cudaFuncSetAttribute(select_hits_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  if (e != cudaSuccess) return vk_err(e);
+  if (sh > TK_SMEM) return VK_E_ARG;
+  int rc = vk_max_smem(select_hits_k, TK_SMEM);
+  if (rc != 0) return rc;
   select_hits_k<<<(unsigned)((n_spec + TK_WARPS - 1) / TK_WARPS), TK_WARPS * 32, sh, (cudaStream_t)stream>>>(
       n_spec, spec_hyp_off, h_lo, h_hi, win_off, hyp_shift, seg_cnt, hit_rc, hit_isum, hyp_scored, hyp_matched, topk,
       pair_closure, partner, cap, list_pow2, key_cap, c_hyp, c_row, c_cnt, c_isum, n_cand, spec_scored,
       spec_matched);
-  const int rc = vk_launch_status();
+  rc = vk_launch_status();
   if (rc != 0) return rc;
   const int big_cap = 2 * list_pow2 > 1024 ? 2 * list_pow2 : 1024;
   const size_t bsh = ((sizeof(BigScratch) + 15) & ~(size_t)15) + (size_t)big_cap * 12 + (size_t)list_pow2 * 16;
-  e = cudaFuncSetAttribute(select_hits_big_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsh);
-  if (e != cudaSuccess) return vk_err(e);
+  rc = vk_max_smem(select_hits_big_k, TK_SMEM);
+  if (rc != 0) return rc;
   select_hits_big_k<<<(unsigned)(n_spec < 592 ? n_spec : 592), HB_WARPS * 32, bsh, (cudaStream_t)stream>>>(
       n_spec, spec_hyp_off, h_lo, h_hi, win_off, hyp_shift, seg_cnt, hit_rc, hit_isum, topk, pair_closure, partner, cap,
       list_pow2, big_cap, c_hyp, c_row, c_cnt, c_isum, n_cand);
