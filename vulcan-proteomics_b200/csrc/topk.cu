@@ -121,11 +121,12 @@ __device__ __forceinline__ uint64_t smem_kth_largest_radix(const uint64_t* key, 
   return prefix;
 }
 
-// Spectra a warp of the launch over the left ones looks at.  A left spectrum keeps its warp for some 50 us, so they are
-// dealt in small groups over many CTAs; 32 at a time by 296 CTAs took 0.65 ms on 40,000 spectra of an index where many
-// partners fall beside the window (masses of a pair that round differently), 8 / 4 / 2 / 1 take 0.320 / 0.286 / 0.295 /
-// 0.319; with none left 0.002 / 0.004 / 0.007 / 0.010 ms.
+// Spectra a warp of the launch over the left ones looks at: one, or 2 or 4 neighbours where one each would be more than
+// TK_REST_CTAS CTAs.  With none left the launch takes 0.004 / 0.007 / 0.010 ms at 4 / 2 / 1 of 40,000; with all left
+// (overlapping windows, 850 rows each) 20,000 spectra take 0.447 ms at 4 a warp and 0.361 at 1, and 2,000 four times as
+// long as at 1.
 constexpr int TK_REST = 4;
+constexpr int TK_REST_CTAS = 8192;
 #ifndef TK_UNROLL
 #define TK_UNROLL 8            // count loads in flight per lane
 #endif
@@ -142,18 +143,24 @@ __device__ __forceinline__ int64_t win_rows(int64_t w0, int64_t lo, int64_t hi, 
 //   1. the counts are read once into a histogram, which gives the count T of the topk-th entry and how many entries
 //      tie at T;
 //   2. a second read (L1 / L2) marks the rows above T, and the last of the tied ones (ties go to the higher row);
-//   3. the partner of every marked row is marked in a second bitmap;
-//   4. the rows of the union come out in order: position by prefix popcounts, count from the marked rows' list.
+//   3. the partner of every marked row is marked in a second bitmap; the few outside their row's window (a pair's
+//      masses differ in the last bits on an index summed sequence by sequence, so a window's edge may part it) are
+//      listed and sorted across the lanes;
+//   4. the rows of the union come out in order: position by prefix popcounts and the listed rows before them, count
+//      from the marked rows' list.
 // 4.2k warp instructions per spectrum of 850 window rows at topk 100, where collecting keys, radix-selecting and
 // sorting them took 10.8k; bound by issue (0.67 a cycle) and the L2 latency of the counts.  Measured per launch,
 // before -> now: 40,000 spectra at topk 100 0.725 -> 0.203 ms, 16,384 with 2,100 window rows each at topk 200
 // 1.588 -> 0.178, 10,001 at topk 500 1.112 -> 0.113, 32 spectra 0.009 -> 0.0064 (and 0.002 for the launch that looks
 // for what was left over).  Staging the rows of step 4 in shared memory for whole-sector writes was slower (0.228 and
-// 0.142: fewer warps per SM), and so was a tally in byte fields of registers (0.216).
-// What does not fit goes to select_topk_k by n_cand = -1: more than 32 hypotheses or overlapping windows, more than
-// TR_WORDS * 32 window rows, a count above 254, a partner outside its own hypothesis' window.
+// 0.142: fewer warps per SM), and so was a tally in byte fields of registers (0.216).  The listed partners: 20,000
+// spectra of 850 window rows at topk 100, all with one, 0.170 ms; leaving such spectra to select_topk_k took 0.517
+// (0.346 without this kernel).
+// What does not fit goes to select_topk_k by n_cand = -1: more than 32 hypotheses or overlapping windows (seen before
+// a count is read), more than TR_WORDS * 32 window rows, a count above 254, more than TR_SIDE partners outside.
 constexpr int TR_WORDS = 384;        // bitmap words per spectrum: 12,288 window rows
 constexpr int TR_TOPK = 512;         // longest list
+constexpr int TR_SIDE = 32;          // partners outside their row's window (one a lane)
 
 struct __align__(16) RowsScratch {   // per warp, the windows in row order
   int64_t lo[32], w0[32];
@@ -322,23 +329,85 @@ select_topk_rows_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   }
   __syncwarp();
   // 3. partners
+  uint64_t* side = reinterpret_cast<uint64_t*>(W.w0);   // (the counts are read) row << 5 | local hypothesis
+  int n_side = 0;                                       // partners outside their row's window
   if (pair_closure) {
-    bool out = false;
-    for (int i = lane; i < n_sel; i += 32) {
-      const uint32_t e = list[i];
-      const int r = (int)(e >> 8) & 31, at = (int)(e >> 13) - 32 * W.word[r];
-      const int64_t p = partner[W.lo[r] + at] - W.lo[r];
-      if (p >= 0 && p < W.n[r]) atomicOr(&W.all[W.word[r] + (int)(p >> 5)], 1u << (p & 31));
-      else out = true;
+    bool bad = false;
+    for (int i0 = 0; i0 < n_sel; i0 += 128) {
+      uint32_t e[4];
+      int64_t p[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {   // the loads first
+        const int i = i0 + 32 * u + lane;
+        e[u] = i < n_sel ? list[i] : 0u;
+        const int r = (int)(e[u] >> 8) & 31;
+        p[u] = i < n_sel ? partner[W.lo[r] + (int)(e[u] >> 13) - 32 * W.word[r]] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (i0 + 32 * u >= n_sel) break;   // uniform
+        const bool mine = i0 + 32 * u + lane < n_sel;
+        const int r = (int)(e[u] >> 8) & 31;
+        const int64_t at = p[u] - W.lo[r];
+        const bool out = mine && (at < 0 || at >= W.n[r]);
+        if (mine && !out) atomicOr(&W.all[W.word[r] + (int)(at >> 5)], 1u << (at & 31));
+        const unsigned m = __ballot_sync(VK_FULL, out);
+        if (m) {
+          const int k = n_side + __popc(m & lt_mask);
+          if (out && k < TR_SIDE) side[k] = ((uint64_t)p[u] << 5) | (uint64_t)W.hl[r];
+          bad |= out && ((uint64_t)p[u] >> 30) != 0ull;
+          n_side += __popc(m);
+        }
+      }
     }
-    if (__any_sync(VK_FULL, out)) {
+    if (n_side > TR_SIDE || __any_sync(VK_FULL, bad)) {
       if (lane == 0) n_cand[s] = -1;
       return;
     }
   }
   __syncwarp();
+  // The outside partners, sorted by (row, hypothesis) across the lanes, one lane per row: a row of the union takes the
+  // lower of the two hypotheses, another is inserted.  place: the word of the union that holds or follows the row;
+  // below: the word's bits before it
+  bool ins = false, lower = false;
+  int side_hl = 0, place = words, rank = 0, n_ins = 0;
+  uint32_t below = 0u;
+  int64_t side_row = 0;
+  if (n_side) {
+    uint64_t k = lane < n_side ? side[lane] : ~0ull;
+    for (int size = 2; size <= 32; size <<= 1)
+      for (int st = size >> 1; st > 0; st >>= 1) {
+        const uint64_t o = __shfl_xor_sync(VK_FULL, k, st);
+        if ((((lane & size) == 0) == ((lane & st) == 0)) ? o < k : o > k) k = o;
+      }
+    const uint64_t before = __shfl_up_sync(VK_FULL, k, 1);
+    const bool head = k != ~0ull && (lane == 0 || (before >> 5) != (k >> 5));
+    side_row = (int64_t)(k >> 5);
+    side_hl = (int)(k & 31);
+    bool found = false, set = false;
+    for (int r = 0; r < nhs && W.n[r] > 0; ++r) {
+      const int64_t at = side_row - W.lo[r];
+      if (!found && at < W.n[r]) {   // the first window that ends behind the row
+        found = true;
+        place = W.word[r];
+        if (at >= 0) {
+          place += (int)(at >> 5);
+          below = (1u << (at & 31)) - 1u;
+          set = (W.all[place] >> (at & 31)) & 1u;
+          lower = head && set && side_hl < W.hl[r];
+        }
+      }
+    }
+    ins = head && !set;
+    const unsigned m = __ballot_sync(VK_FULL, ins);
+    rank = __popc(m & lt_mask);
+    n_ins = __popc(m);
+    if (ins) side[rank] = (uint64_t)side_row;
+    __syncwarp();
+  }
   // 4. the rows of the union, a word per lane
   int carry = 0;   // rows and marked rows before this chunk of words: low and high half
+  int si = 0, side_at = 0;
   const int64_t slot = (int64_t)s * cap;
   for (int w0 = 0; w0 < words; w0 += 32) {
     const int w = w0 + lane;
@@ -347,6 +416,11 @@ select_topk_rows_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
     const int both = __popc(u) | (__popc(m) << 16);
     const int end = vk::warp_incl_scan_i32(both) + carry;
     int at = (end - both) & 0xffff, li = (end - both) >> 16;
+    if (n_side) {
+      const int p_at = __shfl_sync(VK_FULL, at, place & 31);
+      const uint32_t p_u = __shfl_sync(VK_FULL, u, place & 31);
+      if (place >= w0 && place < w0 + 32) side_at = p_at + __popc(p_u & below);
+    }
     int r = 0;
     while (r + 1 < nhs && W.word[r + 1] <= w && W.n[r + 1] > 0) ++r;
     const int64_t h = hb + W.hl[r], row0 = W.lo[r] + 32 * (w - W.word[r]);
@@ -355,18 +429,29 @@ select_topk_rows_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
       u &= u - 1u;
       int c = -1;
       if ((m >> b) & 1u) c = (int)(list[li++] & 255u);
-      c_hyp[slot + at] = h;
-      c_row[slot + at] = row0 + b;
-      c_cnt[slot + at] = c;
+      while (si < n_ins && (int64_t)side[si] < row0 + b) ++si;   // rows inserted before this one
+      c_hyp[slot + at + si] = h;
+      c_row[slot + at + si] = row0 + b;
+      c_cnt[slot + at + si] = c;
       ++at;
     }
     carry = __shfl_sync(VK_FULL, end, 31);
   }
-  if (lane == 0) n_cand[s] = carry & 0xffff;
+  const int n_union = carry & 0xffff;
+  if (n_side) {
+    __syncwarp();   // the rows' hypotheses are written before they are lowered
+    const int64_t at = slot + (place < words ? side_at : n_union) + rank;
+    if (ins) {
+      c_row[at] = side_row;
+      c_cnt[at] = -1;
+    }
+    if (ins || lower) c_hyp[at] = hb + side_hl;
+  }
+  if (lane == 0) n_cand[s] = n_union + n_ins;
 }
 
 // ------------------------------------------------------------------------------------------ any windows
-// One spectrum per warp; rest: only the spectra select_topk_rows_k left (n_cand = -1).
+// One spectrum per warp; rest > 0: only the spectra select_topk_rows_k left (n_cand = -1), rest neighbours per warp.
 __global__ void __launch_bounds__(TK_WARPS * 32)
 select_topk_k(int n_spec, int rest, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
               const int64_t* win_off,
@@ -541,8 +626,8 @@ select_topk_k(int n_spec, int rest, const int64_t* spec_hyp_off, const int64_t* 
     for (int s = first; s < n_spec; s += step) one(s);
     return;
   }
-  for (int s0 = first * TK_REST; s0 < n_spec; s0 += step * TK_REST) {
-    unsigned left = __ballot_sync(VK_FULL, lane < TK_REST && s0 + lane < n_spec && n_cand[s0 + lane] < 0);
+  for (int s0 = first * rest; s0 < n_spec; s0 += step * rest) {
+    unsigned left = __ballot_sync(VK_FULL, lane < rest && s0 + lane < n_spec && n_cand[s0 + lane] < 0);
     for (; left; left &= left - 1u) one(s0 + __ffs(left) - 1);
   }
 }
@@ -1270,8 +1355,8 @@ int vk_select_topk(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   if (rc != 0) return rc;
   const unsigned blocks = (unsigned)((n_spec + TK_WARPS - 1) / TK_WARPS);
   unsigned grid = blocks;
-  const int rest = topk_by_rows(thr, topk);
-  if (rest) {
+  int rest = 0;
+  if (topk_by_rows(thr, topk)) {
     const int list_len = ((topk > 256 ? topk : 256) + 3) & ~3;   // each warp's scratch on a 16-byte boundary
     const size_t rsh = (sizeof(RowsScratch) + (size_t)list_len * 4) * TK_WARPS;
     rc = vk_max_smem(select_topk_rows_k, (sizeof(RowsScratch) + (size_t)TR_TOPK * 4) * TK_WARPS);
@@ -1281,7 +1366,8 @@ int vk_select_topk(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
         c_hyp, c_row, c_cnt, n_cand, hyp_scored, hyp_matched, spec_scored, spec_matched);
     rc = vk_launch_status();
     if (rc != 0) return rc;
-    grid = (unsigned)((n_spec + TK_WARPS * TK_REST - 1) / (TK_WARPS * TK_REST));
+    for (rest = 1; rest < TK_REST && (n_spec + TK_WARPS * rest - 1) / (TK_WARPS * rest) > TK_REST_CTAS;) rest <<= 1;
+    grid = (unsigned)((n_spec + TK_WARPS * rest - 1) / (TK_WARPS * rest));
   }
   select_topk_k<<<grid, TK_WARPS * 32, sh, (cudaStream_t)stream>>>(
       n_spec, rest, spec_hyp_off, h_lo, h_hi, win_off, cnt, cnt_cap, partner, thr, topk, pair_closure, cap, list_pow2,
