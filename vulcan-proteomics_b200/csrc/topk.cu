@@ -777,6 +777,67 @@ __device__ __forceinline__ void finish_hits(int lane, int s, int64_t hb, int n_s
   if (lane == 0) n_cand[s] = n_out;
 }
 
+// The hits of a spectrum that are more than shared memory holds, by the warp that saw that, in one more visit: keys and
+// hit slots are collected in the order they come (S.hyp holds the hypotheses' order when by_rank), and when the next
+// batch has no room the topk largest stay, in order, and only larger ones enter from then on.  Returns how many are
+// held at the end, the topk largest among them.  Bound by the latency of the visit and of the selections, some 20 us
+// each, of which a list of 600 to 1,200 hits takes two.
+__device__ __forceinline__ int stream_hits(HitScratch& S, uint64_t* key, uint32_t* src, uint32_t* hist, int cap,
+                                               int topk, bool by_rank, int nhs, int64_t hb, const int64_t* h_lo,
+                                               const int64_t* h_hi, const int64_t* win_off, const int8_t* hyp_shift,
+                                               const uint32_t* seg_cnt, const uint64_t* rc, int64_t w_base) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  int n = 0;
+  uint64_t floor = 0ull;
+  for (int g0 = 0; g0 < nhs; g0 += 32) {
+    __syncwarp();
+    if (!by_rank && lane < min(32, nhs - g0)) S.hyp[lane] = g0 + lane;
+    __syncwarp();
+    gather_hits(S, min(32, nhs - g0), hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane,
+                [&](bool ok, int64_t pos, uint64_t v, int hl) {
+      const uint64_t k = ok ? sel_key(hit_count(v), hit_row(v), hl) : 0ull;
+      unsigned m = __ballot_sync(VK_FULL, ok && k >= floor);
+      if (n + __popc(m) > cap) {
+        __syncwarp();
+        floor = smem_kth_largest(key, n, topk, hist, lane);
+        int kept = 0;
+        for (int i0 = 0; i0 < n; i0 += 32) {
+          const int i = i0 + lane;
+          const uint64_t x = i < n ? key[i] : 0ull;
+          const uint32_t p = i < n ? src[i] : 0u;
+          const bool take = i < n && x >= floor;
+          const unsigned t = __ballot_sync(VK_FULL, take);
+          __syncwarp();   // every read of the group before its writes
+          if (take) {
+            key[kept + __popc(t & lt_mask)] = x;
+            src[kept + __popc(t & lt_mask)] = p;
+          }
+          kept += __popc(t);
+          __syncwarp();
+        }
+        n = kept;
+        m = __ballot_sync(VK_FULL, ok && k >= floor);
+      }
+      if ((m >> lane) & 1u) {
+        key[n + __popc(m & lt_mask)] = k;
+        src[n + __popc(m & lt_mask)] = (uint32_t)(pos - w_base);
+      }
+      n += __popc(m);
+    });
+  }
+  __syncwarp();
+  return n;
+}
+
+// Whether a spectrum with more hits than shared memory holds is left to a CTA: windows of at least `most` rows.
+__device__ __forceinline__ bool leave_hits(int64_t hb, int nhs, const int64_t* h_lo, const int64_t* h_hi, int64_t most,
+                                           int lane) {
+  long long rows = 0;
+  for (int h = lane; h < nhs; h += 32) rows += max(h_hi[hb + h] - h_lo[hb + h], (int64_t)0);
+  return vk::warp_sum(rows) >= most;
+}
+
 // Shortlist from the hit lists of vk_k1_hits, one warp per spectrum: the hits of the spectrum's hypotheses ranked by
 // (count desc, row desc, hypothesis asc) with the keys of select_topk_k, the first topk kept (all when fewer),
 // optionally with pair closure, sorted by (row, hypothesis), duplicate rows merged to the lowest hypothesis (its
@@ -784,15 +845,23 @@ __device__ __forceinline__ void finish_hits(int lane, int s, int64_t hb, int n_s
 //   Fast path (no closure, at most 32 hypotheses, their windows pairwise disjoint -- the usual case): the hypotheses
 //   are visited in window order and each one's hits come in row order, so the collected hits are already sorted by
 //   row with no duplicates; selection keeps that order and no sort is needed.
-//   Otherwise: collect, select, add partners, bitonic sort and merge.  Spectra with more hits than shared memory
-//   holds are left to select_hits_big_k (n_cand = -1), as soon as that is seen.
-__global__ void __launch_bounds__(TK_WARPS * 32)
+//   Otherwise: collect, select, add partners, bitonic sort and merge.
+// When more hits come than shared memory holds, the warp begins again with stream_hits or, where the windows span
+// big_rows rows or more, leaves the spectrum to select_hits_big_k (n_cand = -1): a CTA has a list done sooner than a
+// warp, but 592 run at once instead of some 2,400, and its last step is one warp's.  Per launch, CTA / warp: 20,000
+// spectra of 603 hits at topk 100 2.86 / 0.39 ms (an eight-pass radix select in global memory took 1.07), 2,000 of
+// 5,070 0.54 / 0.20; 500 of 1,206 0.102 / 0.084, of 5,070 0.135 / 0.187; 32 of 603 0.056 / 0.058, of 1,206 0.062 /
+// 0.082.  Hence big_rows (twice the hits there): 1,024 up to an SM a spectrum, 4,096 up to a CTA each, 16,384 up to two
+// spectra a CTA, else 65,536.
+// At least 4 CTAs an SM: left to itself the compiler keeps to 56 registers and spills (5% on lists that fit).
+__global__ void __launch_bounds__(TK_WARPS * 32, 4)
 select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
               const int64_t* win_off, const int8_t* hyp_shift, const uint32_t* seg_cnt, const uint64_t* rc,
               const uint32_t* hit_isum,
               const uint32_t* hyp_scored, const uint64_t* hyp_matched, int topk, int pair_closure,
-              const int64_t* partner, int cap, int list_pow2, int key_cap, int64_t* c_hyp, int64_t* c_row,
-              int64_t* c_cnt, uint32_t* c_isum, int64_t* n_cand, int64_t* spec_scored, int64_t* spec_matched) {
+              const int64_t* partner, int cap, int list_pow2, int key_cap, int64_t big_rows, int64_t* c_hyp,
+              int64_t* c_row, int64_t* c_cnt, uint32_t* c_isum, int64_t* n_cand, int64_t* spec_scored,
+              int64_t* spec_matched) {
   extern __shared__ __align__(16) uint8_t tk_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int s = blockIdx.x * TK_WARPS + warp;
@@ -824,7 +893,6 @@ select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, cons
     spec_scored[s] = sc;
     spec_matched[s] = mt;
   }
-  // ---------------------------------------------------------------- fast path
   bool fast = !pair_closure && nhs <= 32;
   int my_rank = 0;
   if (fast) {
@@ -844,57 +912,16 @@ select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, cons
     }
     fast = !__any_sync(VK_FULL, overlap);
   }
+  // the hits, as many as shared memory holds: the hypotheses in window order (fast) or 32 at a time in index order
   if (fast) {
-    long long n_app = 0;
     __syncwarp();
-    if (lane < nhs) S.hyp[my_rank] = lane;     // the hypotheses in window order
+    if (lane < nhs) S.hyp[my_rank] = lane;
     __syncwarp();
-    gather_hits(S, nhs, hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane,
-                [&](bool ok, int64_t pos, uint64_t v, int hl_) {
-      const unsigned m = __ballot_sync(VK_FULL, ok);
-      const long long at = n_app + __popc(m & lt_mask);
-      if (ok && at < key_cap) {
-        key[at] = sel_key(hit_count(v), hit_row(v), hl_);
-        src[at] = (uint32_t)(pos - w_base);
-      }
-      n_app += __popc(m);
-    }, [&]() { return n_app <= key_cap; });
-    __syncwarp();
-    if (n_app > key_cap) {   // more than shared memory holds: select_hits_big_k
-      if (lane == 0) n_cand[s] = -1;
-      return;
-    }
-    {
-      const int n_k = (int)n_app;
-      const bool limit = n_k > topk;
-      const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, hist, lane) : 0ull;
-      int n_out = 0;
-      for (int i0 = 0; i0 < n_k; i0 += 32) {
-        const int i = i0 + lane;
-        const uint64_t k = i < n_k ? key[i] : 0ull;
-        const bool take = i < n_k && (!limit || k >= kth);
-        const unsigned m = __ballot_sync(VK_FULL, take);
-        if (take) {
-          const int64_t pos = w_base + src[i];
-          const uint64_t v = rc[pos];
-          const int64_t at = slot + n_out + __popc(m & lt_mask);
-          c_hyp[at] = hb + ((1 << 18) - 1 - (int)(k & 0x3ffff));
-          c_row[at] = hit_row(v);
-          c_cnt[at] = hit_count(v);
-          if (c_isum) c_isum[at] = hit_isum[pos];
-        }
-        n_out += __popc(m);
-      }
-      if (lane == 0) n_cand[s] = n_out;
-      return;
-    }
   }
-
-  // ---------------------------------------------------------------- general path
   long long n_app = 0;
-  for (int g0 = 0; g0 < nhs && n_app <= key_cap; g0 += 32) {   // 32 hypotheses at a time, in index order
+  for (int g0 = 0; g0 < nhs && n_app <= key_cap; g0 += 32) {
     __syncwarp();
-    if (lane < min(32, nhs - g0)) S.hyp[lane] = g0 + lane;
+    if (!fast && lane < min(32, nhs - g0)) S.hyp[lane] = g0 + lane;
     __syncwarp();
     gather_hits(S, min(32, nhs - g0), hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc, lane,
                 [&](bool ok, int64_t pos, uint64_t v, int hl_) {
@@ -908,12 +935,41 @@ select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, cons
     }, [&]() { return n_app <= key_cap; });
   }
   __syncwarp();
-  if (n_app > key_cap) {   // more than shared memory holds: select_hits_big_k
-    if (lane == 0) n_cand[s] = -1;
-    return;
+  if (n_app > key_cap) {   // more than it holds
+    if (leave_hits(hb, nhs, h_lo, h_hi, big_rows, lane)) {
+      if (lane == 0) n_cand[s] = -1;
+      return;
+    }
+    n_app = stream_hits(S, key, src, hist, key_cap, topk, fast, nhs, hb, h_lo, h_hi, win_off, hyp_shift, seg_cnt, rc,
+                        w_base);
   }
   const int n_k = (int)n_app;
   const bool limit = n_k > topk;
+  // ---------------------------------------------------------------- fast path
+  if (fast) {
+    const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, hist, lane) : 0ull;
+    int n_out = 0;
+    for (int i0 = 0; i0 < n_k; i0 += 32) {
+      const int i = i0 + lane;
+      const uint64_t k = i < n_k ? key[i] : 0ull;
+      const bool take = i < n_k && (!limit || k >= kth);
+      const unsigned m = __ballot_sync(VK_FULL, take);
+      if (take) {
+        const int64_t pos = w_base + src[i];
+        const uint64_t v = rc[pos];
+        const int64_t at = slot + n_out + __popc(m & lt_mask);
+        c_hyp[at] = hb + ((1 << 18) - 1 - (int)(k & 0x3ffff));
+        c_row[at] = hit_row(v);
+        c_cnt[at] = hit_count(v);
+        if (c_isum) c_isum[at] = hit_isum[pos];
+      }
+      n_out += __popc(m);
+    }
+    if (lane == 0) n_cand[s] = n_out;
+    return;
+  }
+
+  // ---------------------------------------------------------------- general path
   int n_sel = 0;
   const uint64_t kth = limit ? smem_kth_largest(key, n_k, topk, hist, lane) : 0ull;
   for (int i0 = 0; i0 < n_k; i0 += 32) {
@@ -944,10 +1000,10 @@ select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, cons
 // hits above it are collected as keys and the exact topk-th is selected among them, and one warp finishes the list.
 // What bounds it is the latency of the dependent reads (segment count, hit) of a visit.  A warp per spectrum ran an
 // eight-pass radix select over the lists and two more visits, each some 140 us for 20,000 hits; 777 spectra with open
-// windows: 1.41 ms before, 0.22 now (0.049 of it select_hits_k); 4,000 spectra of which one in five holds more than
-// 512 hits: 0.146 before, 0.142 now.  8 and 4 warps per CTA: 0.25 and 0.31 on the open windows.  Warps that take whole
-// groups of segments instead of a share of each group's hits: 0.20, but 0.170 on the 4,000 (one group each).
+// windows: 1.41 ms before, 0.22 now (0.049 of it select_hits_k).  8 and 4 warps per CTA: 0.25 and 0.31.  Warps that
+// take whole groups of segments instead of a share of each group's hits: 0.20, but slower on lists of one group.
 constexpr int HB_WARPS = 16;
+constexpr int HB_FEW = 148;         // spectra that have an SM each
 constexpr int HB_COUNTS = 1024;     // histogram bins of the counts; the last holds all larger ones
 
 struct BigScratch {
@@ -1415,7 +1471,12 @@ int vk_select_hits(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   }
   int list_pow2 = 32;
   while (list_pow2 < (pair_closure ? 2 : 1) * topk) list_pow2 <<= 1;
-  const int key_cap = list_pow2 > 512 ? list_pow2 : 512;
+  int key_cap = list_pow2 > 512 ? list_pow2 : 512;
+  if (key_cap < topk + 128) key_cap *= 2;   // room for new hits beside the topk that stay
+  const int64_t big_rows = n_spec <= HB_FEW       ? 1024      // (see select_hits_k)
+                           : n_spec <= 4 * HB_FEW ? 4096
+                           : n_spec <= 8 * HB_FEW ? 16384
+                                                  : 65536;
   const size_t per_warp = (size_t)key_cap * 12 + (size_t)list_pow2 * 16 + 1024 + sizeof(HitScratch);
   const size_t sh = per_warp * TK_WARPS;
   if (sh > TK_SMEM) return VK_E_ARG;
@@ -1423,7 +1484,7 @@ int vk_select_hits(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   if (rc != 0) return rc;
   select_hits_k<<<(unsigned)((n_spec + TK_WARPS - 1) / TK_WARPS), TK_WARPS * 32, sh, (cudaStream_t)stream>>>(
       n_spec, spec_hyp_off, h_lo, h_hi, win_off, hyp_shift, seg_cnt, hit_rc, hit_isum, hyp_scored, hyp_matched, topk,
-      pair_closure, partner, cap, list_pow2, key_cap, c_hyp, c_row, c_cnt, c_isum, n_cand, spec_scored,
+      pair_closure, partner, cap, list_pow2, key_cap, big_rows, c_hyp, c_row, c_cnt, c_isum, n_cand, spec_scored,
       spec_matched);
   rc = vk_launch_status();
   if (rc != 0) return rc;
