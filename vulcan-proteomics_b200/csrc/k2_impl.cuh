@@ -232,9 +232,9 @@ __device__ __forceinline__ K2Val k2_score(const SmemFrag& fp, const PT& pt, int 
 
 // ------------------------------------------------------------------------------------------ dense lists, closed
 //
-// One CTA of KD_WARPS warps per spectrum at a time, one lane per candidate.  Most
-// ions of a candidate meet no peak, and the lanes that do meet one differ from ion to ion, so a warp takes its
-// candidates in two loops instead of one lookup per ion:
+// One CTA of KD_WARPS warps per spectrum at a time, one lane per candidate.  Most ions of a candidate meet no peak, and
+// the lanes that do meet one differ from ion to ion, so a warp takes its candidates in two loops instead of one lookup
+// per ion:
 //   * walk (the ion index uniform over the warp): the running f32 masses of the b and y ions, each tested with one
 //     fused multiply-add and one bit of a presence bitmap (KD_BITS buckets of 1/KD_SCALE Th, wrapping around; a peak
 //     sets every bucket from which an ion could reach it, so a clear bit means no peak in the ion's window); the
@@ -243,9 +243,16 @@ __device__ __forceinline__ K2Val k2_score(const SmemFrag& fp, const PT& pt, int 
 //     peak by a table of start indices, most intense peak, its ppm term; then every lane adds its own ions' results,
 //     b then y in ion order.  The arithmetic is k2_score's, so the outputs are bit-identical to it.
 // Residues come four at a time from aligned words (single bytes at the ends of the table), their masses
-// from one table of mono + delta, lnfact of small counts from a table built by the same function.  A
-// candidate of more than KD_MAXLEN residues, or with more marked ions than its lists hold, is scored by k2_score;
-// with fragment charges above 1 each lane looks its own ions up, charge by charge.
+// from one table of mono + delta, lnfact of small counts from a table built by the same function.  With fragment
+// charges above 1 each lane looks its own ions up, charge by charge.
+//   * left: a candidate of more than KD_MAXLEN residues, or with more marked ions than its lists hold, is scored when
+//     the warp's others are: one at a time by the whole warp (kd_score_warp), or by k2_score side by side where more
+//     than KD_SLOW of 32 are.  A spectrum of at most KD_FEW candidates takes a warp for each from the start.  Both
+//     because a lane that scores alone leaves 31 idle for some 50 us, and an SM holds 24 of these warps.  Measured,
+//     left to a lane each -> now: 3,000 spectra of 2 rows of 70-119 residues 0.211 -> 0.046 ms, of 8 0.248 -> 0.173, of
+//     40 0.359 -> 0.357; 8 rows of 50-65 residues at fragment charges up to 3 0.310 -> 0.166, 300 1.95 -> 0.93; 20,000
+//     spectra of 2 usual rows 0.113 -> 0.105, at charges up to 3 0.166 -> 0.134.  14 for KD_SLOW: 0.244 for 12 rows of
+//     70-119 residues instead of 0.265, but 0.269 for 40 rows of 50-65 at 0.5 Da instead of 0.242.
 //
 // What bounds it: instruction issue and the latency of a warp's dependent steps (0.6 instructions a cycle; HBM is at
 // 5%).  Of 0.341 ms for 20,000 spectra (3.0M candidates) the tables take 0.09 when nothing hides them, the walk 0.13,
@@ -264,6 +271,9 @@ constexpr int KD_BITS = 8192;        // presence buckets
 constexpr float KD_SCALE = 4.0f;     // buckets per Th: 2,048 Th before they wrap
 constexpr int KD_LNF = 32;           // tabulated lnfact arguments
 constexpr int KD_MAXLEN = 65;        // residues whose 64 ions fit a mask
+constexpr int KD_FEW = KD_WARPS;     // candidates of a spectrum that take a warp each
+constexpr int KD_SLOW = 8;           // of 32 candidates, those left that the warp takes one after another
+constexpr int16_t KD_LEFT = -1;      // the longest run of a candidate that is left
 constexpr int KD_QUEUE = 256;        // ions looked up per round of a warp (a lane has at most 2 * KD_LIST)
 static_assert(KD_QUEUE >= 2 * KD_LIST, "a lane's ions fit a round");
 
@@ -388,6 +398,56 @@ static __device__ __noinline__ K2Val kd_score_serial(const SmemFrag* fp, const K
   return k2_score<false, DensePeaks>(*fp, pt, r, maxfz, seq_off, len, mask, mass32, res, tol_lo, tol_hi, 0.f);
 }
 
+// One candidate by the whole warp: its ion masses summed by two lanes, the ions of every charge looked up 32 at a time,
+// the matches added up in k2_score's order.  Every lane returns the candidate's values.
+static __device__ __noinline__ K2Val kd_score_warp(const SmemFrag* fp, K2DenseSmem* S, int warp, uint32_t q0,
+                                                   const uint8_t* seq, int len, int maxfz, uint64_t mask, float mass,
+                                                   float tol_lo, float tol_hi) {
+  const int lane = threadIdx.x & 31, n = len - 1, nz = maxfz - 1, half = n * nz;
+  K2Val v{0.f, 0.f, 0.f, 0, 0, 0, 0};
+  if (n <= 0 || nz <= 0) return v;
+  float* rm = &S->ion[warp][0][0][0];   // n <= 254 residue masses, then the b and the y ions
+  float* ions = rm + 256;
+  for (int k = lane; k < n; k += 32) rm[k] = resmass(*fp, seq[k], k, mask);
+  __syncwarp();
+  if (lane < 2) {
+    const float nt = nterm_of(*fp, mask), sign = lane ? -1.f : 1.f;
+    float c = lane ? __fsub_rn(mass, nt) : nt;
+    float* to = ions + 256 * lane;
+#pragma unroll 4
+    for (int k = 0; k < n; ++k) to[k] = c = __fadd_rn(c, __fmul_rn(sign, rm[k]));   // (x - r is x + -r)
+  }
+  __syncwarp();
+  RunLen rb = {0, 0, 0, 0}, ry = {0, 0, 0, 0};
+  for (int t0 = 0; t0 < 2 * half; t0 += 32) {
+    const int t = t0 + lane, kind = t >= half, i = t - kind * half, k = i / nz, z = i - k * nz + 1;
+    float2 peak = make_float2(0.f, CUDART_NAN_F);
+    float term = 0.f;
+    if (t < 2 * half) {
+      const float base = ions[256 * kind + k], mz = z == 1 ? base : __fdiv_rn(base, (float)z);
+      peak = kd_match(*S, q0, mz, tol_lo, tol_hi, fp->tol_da);
+      term = kd_term(mz, peak);
+    }
+    for (unsigned hit = __ballot_sync(VK_FULL, peak.y >= 0.f); hit; hit &= hit - 1u) {
+      const int l = __ffs(hit) - 1, at = __shfl_sync(VK_FULL, kind << 16 | k, l);
+      const float pint = __shfl_sync(VK_FULL, peak.y, l);
+      v.ppm = __fadd_rn(v.ppm, __shfl_sync(VK_FULL, term, l));
+      if (at >> 16) {
+        v.my += 1;
+        v.sy = __fadd_rn(v.sy, pint);
+        run_matched(ry, at & 0xffff);
+      } else {
+        v.mb += 1;
+        v.sb = __fadd_rn(v.sb, pint);
+        run_matched(rb, at);
+      }
+    }
+  }
+  v.lb = rb.longest;
+  v.ly = ry.longest;
+  return v;
+}
+
 __device__ __forceinline__ double kd_lnfact(const K2DenseSmem& S, int n) {
   return n < KD_LNF ? S.lnf[n] : lnfact(n);
 }
@@ -478,7 +538,7 @@ struct DenseRow {
   const uint8_t* seq;
   uint64_t mask;
   float mass;
-  int row, len, maxfz;
+  int len, maxfz;
 
   // ions to walk; none of an empty row (whose offset may lie anywhere: its residues are not looked at)
   __device__ __forceinline__ int ions() const { return len <= KD_MAXLEN && maxfz > 1 ? max(len - 1, 0) : 0; }
@@ -488,12 +548,12 @@ __device__ __forceinline__ DenseRow kd_row(int64_t c, const int32_t* c_row, cons
                                            const int64_t* seq_off, const uint8_t* len, const uint64_t* mask,
                                            const float* mass32, const uint8_t* res) {
   DenseRow d;
-  d.row = c_row[c];
+  const int row = c_row[c];
   d.maxfz = c_maxfz[c];
-  d.seq = res + seq_off[d.row];
-  d.len = len[d.row];
-  d.mask = mask[d.row];
-  d.mass = mass32[d.row];
+  d.seq = res + seq_off[row];
+  d.len = len[row];
+  d.mask = mask[row];
+  d.mass = mass32[row];
   return d;
 }
 
@@ -507,12 +567,10 @@ __device__ __forceinline__ void kd_begin(RowWords& w, const DenseRow& d, bool li
   if (live && d.ions() > 0) w.begin(res, d.seq, d.len, reinterpret_cast<const uint8_t*>(last));
 }
 
-// Scores the warp's candidates (lanes with `live` hold one each).
-__device__ __forceinline__ void kd_score(K2DenseSmem& S, const DensePeaks& pt, int warp, int lane, bool live,
-                                         const DenseRow& d, RowWords& w, const SmemFrag& fp, const int64_t* seq_off,
-                                         const uint8_t* len, const uint64_t* mask, const float* mass32,
-                                         const uint8_t* res, float tol_lo, float tol_hi, const K2Out& out,
-                                         int64_t c) {
+// Scores the warp's candidates (lanes with `live` hold one each).  True in lanes whose candidate is left to kd_left.
+__device__ __forceinline__ bool kd_score(K2DenseSmem& S, const DensePeaks& pt, int warp, int lane, bool live,
+                                         const DenseRow& d, RowWords& w, const SmemFrag& fp, float tol_lo, float tol_hi,
+                                         const K2Out& out, int64_t c) {
   const bool fits = live && d.len <= KD_MAXLEN;
   const int n_ion = live ? d.ions() : 0;
   const int n_max = __reduce_max_sync(VK_FULL, n_ion);
@@ -572,9 +630,10 @@ __device__ __forceinline__ void kd_score(K2DenseSmem& S, const DensePeaks& pt, i
       __syncwarp();
     }
   }
-  if (!live) return;
+  if (!live) return false;
   if (!fits || over) {
-    v = kd_score_serial(&fp, &S, pt.np, pt.q0, d.row, d.maxfz, seq_off, len, mask, mass32, res, tol_lo, tol_hi);
+    out.lb[c] = KD_LEFT;
+    return true;
   } else {
     if (z_max > 2) {
       uint64_t todo = mark_b;
@@ -612,6 +671,36 @@ __device__ __forceinline__ void kd_score(K2DenseSmem& S, const DensePeaks& pt, i
     v.ly = kd_longest(hit_y);
   }
   k2_write(v, [&](int n) { return kd_lnfact(S, n); }, out, c);
+  return false;
+}
+
+// The candidates that the walk does not score.  few: the spectrum's, a warp each; else those of the warp that kd_score
+// left, one after another by the whole warp where few of 32 are, side by side otherwise.
+__device__ __forceinline__ void kd_left(const SmemFrag* fp, K2DenseSmem* S, int np, uint32_t q0, int warp, bool few,
+                                            int64_t c0, int64_t c1, const int32_t* c_row, const int8_t* c_maxfz,
+                                            const int64_t* seq_off, const uint8_t* len, const uint64_t* mask,
+                                            const float* mass32, const uint8_t* res, float tol_lo, float tol_hi,
+                                            const K2Out out) {
+  const int lane = threadIdx.x & 31, width = few ? 1 : 32;
+  for (int64_t cw = c0 + warp * width; cw < c1; cw += KD_WARPS * width) {
+    const int64_t c = cw + lane;
+    const bool mine = lane < width && c < c1 && (few || out.lb[c] == KD_LEFT);
+    unsigned todo = __ballot_sync(VK_FULL, mine);
+    if (!todo) continue;
+    K2Val v{0.f, 0.f, 0.f, 0, 0, 0, 0};
+    if (__popc(todo) <= KD_SLOW) {
+      for (; todo; todo &= todo - 1u) {
+        const int l = __ffs(todo) - 1, r = c_row[cw + l];
+        const K2Val one = kd_score_warp(fp, S, warp, q0, res + seq_off[r], len[r], c_maxfz[cw + l], mask[r], mass32[r],
+                                        tol_lo, tol_hi);
+        if (lane == l) v = one;
+      }
+    } else if (mine) {
+      v = kd_score_serial(fp, S, np, q0, c_row[c], c_maxfz[c], seq_off, len, mask, mass32, res, tol_lo, tol_hi);
+    }
+    if (mine) k2_write(v, [&](int n) { return kd_lnfact(*S, n); }, out, c);
+    __syncwarp();
+  }
 }
 
 // CTA-per-spectrum driver of the closed scoring.  spec_ids == nullptr: spectrum bs uses peaks of spectrum bs.
@@ -668,14 +757,19 @@ __device__ __forceinline__ void k2_dense_body(K2DenseSmem& S, const SmemFrag& fp
     RowWords w{};
     kd_begin(w, d, some, res);
     __syncthreads();
-    for (int64_t cw = c0 + warp * 32; cw < c1; cw += NT) {   // uniform over the warp
+    const bool few = c1 - c0 <= KD_FEW;
+    bool left = few;
+    for (int64_t cw = c0 + warp * 32; cw < c1 && !few; cw += NT) {   // uniform over the warp
       const int64_t c = cw + lane;
-      kd_score(S, pt, warp, lane, c < c1, d, w, fp, seq_off, len, mask, mass32, res, tol_lo, tol_hi, out, c);
+      left |= kd_score(S, pt, warp, lane, c < c1, d, w, fp, tol_lo, tol_hi, out, c);
       __syncwarp();
       const bool more = c + NT < c1;
       if (more) d = kd_row(c + NT, c_row, c_maxfz, seq_off, len, mask, mass32, res);
       kd_begin(w, d, more, res);
     }
+    if (__any_sync(VK_FULL, left))
+      kd_left(&fp, &S, np, pt.q0, warp, few, c0, c1, c_row, c_maxfz, seq_off, len, mask, mass32, res, tol_lo, tol_hi,
+              out);
   }
 }
 
