@@ -247,19 +247,20 @@ __device__ __forceinline__ K2Val k2_score(const SmemFrag& fp, const PT& pt, int 
 // charges above 1 each lane looks its own ions up, charge by charge.
 //   * left: a candidate of more than KD_MAXLEN residues, or with more marked ions than its lists hold, is scored when
 //     the warp's others are: one at a time by the whole warp (kd_score_warp), or by k2_score side by side where more
-//     than KD_SLOW of 32 are.  A spectrum of at most KD_FEW candidates takes a warp for each from the start.  Both
-//     because a lane that scores alone leaves 31 idle for some 50 us, and an SM holds 24 of these warps.  Measured,
-//     left to a lane each -> now: 3,000 spectra of 2 rows of 70-119 residues 0.211 -> 0.046 ms, of 8 0.248 -> 0.173, of
-//     40 0.359 -> 0.357; 8 rows of 50-65 residues at fragment charges up to 3 0.310 -> 0.166, 300 1.95 -> 0.93; 20,000
-//     spectra of 2 usual rows 0.113 -> 0.105, at charges up to 3 0.166 -> 0.134.  14 for KD_SLOW: 0.244 for 12 rows of
-//     70-119 residues instead of 0.265, but 0.269 for 40 rows of 50-65 at 0.5 Da instead of 0.242.
+//     than KD_SLOW of 32 are, because a lane that scores alone leaves 31 idle for some 50 us, and an SM holds 24 of
+//     these warps.  Measured, left to a lane each -> now: 3,000 spectra of 2 rows of 70-119 residues 0.211 -> 0.064 ms,
+//     of 8 0.248 -> 0.172, of 40 0.359 -> 0.357; 8 rows of 50-65 residues at fragment charges up to 3 0.310 -> 0.166,
+//     300 1.95 -> 0.93.  14 for KD_SLOW: 0.244 for 12 rows of 70-119 residues instead of 0.265, but 0.269 for 40 rows
+//     of 50-65 at 0.5 Da instead of 0.242.  A warp for each candidate of spectra of up to 3, without the walk: 8-20%
+//     faster where all spectra are such, but 0.334 ms instead of 0.289 where they have 2 to 6 (two codes on an SM).
 //
-// What bounds it: instruction issue and the latency of a warp's dependent steps (0.6 instructions a cycle; HBM is at
-// 5%).  Of 0.341 ms for 20,000 spectra (3.0M candidates) the tables take 0.09 when nothing hides them, the walk 0.13,
-// the lookup 0.08, the hyperscore and the outputs 0.04.  The warp-per-spectrum kernel with a lookup per ion before it
-// ran 4,700 instructions per 32 candidates at 20.7 active lanes; this one runs 1,900 at 25.  Measured (device time per
-// launch, before -> now): 5.92M candidates of 40,000 spectra 1.590 -> 0.645 ms, 10,001 spectra of up to 1,000
-// candidates at 20 ppm 1.412 -> 0.324, fragment charges up to 3 1.078 -> 0.308, 32 spectra 0.030 -> 0.0096.
+// What bounds it: instruction issue and the latency of a warp's dependent steps (0.54 instructions a cycle and
+// scheduler; HBM is at 15% with cold caches).  Of 0.341 ms for 20,000 spectra (3.0M candidates) the tables take 0.09
+// when nothing hides them, the walk 0.13, the lookup 0.08, the hyperscore and the outputs 0.04.  The warp-per-spectrum
+// kernel with a lookup per ion before it ran 4,700 instructions per 32 candidates at 20.7 active lanes; this one runs
+// 2,100 at 25.6.  Measured (device time per launch, before -> now): 5.92M candidates of 40,000 spectra 1.590 -> 0.645
+// ms, 10,001 spectra of up to 1,000 candidates at 20 ppm 1.412 -> 0.324, fragment charges up to 3 1.078 -> 0.308, 32
+// spectra 0.030 -> 0.0096.
 // 3 warps per CTA at 8 CTAs per SM: 2, 4 and 6 warps took 12-16% longer on the 40,000 spectra (a spectrum's 148
 // candidates are 4.6 warps' worth; wider CTAs idle in their second round, narrower ones build the table with fewer).
 // Testing an ion's charges right after its mass, instead of four ions at a time, cost the overlap of the tests (0.70
@@ -271,7 +272,6 @@ constexpr int KD_BITS = 8192;        // presence buckets
 constexpr float KD_SCALE = 4.0f;     // buckets per Th: 2,048 Th before they wrap
 constexpr int KD_LNF = 32;           // tabulated lnfact arguments
 constexpr int KD_MAXLEN = 65;        // residues whose 64 ions fit a mask
-constexpr int KD_FEW = KD_WARPS;     // candidates of a spectrum that take a warp each
 constexpr int KD_SLOW = 8;           // of 32 candidates, those left that the warp takes one after another
 constexpr int16_t KD_LEFT = -1;      // the longest run of a candidate that is left
 constexpr int KD_QUEUE = 256;        // ions looked up per round of a warp (a lane has at most 2 * KD_LIST)
@@ -674,17 +674,16 @@ __device__ __forceinline__ bool kd_score(K2DenseSmem& S, const DensePeaks& pt, i
   return false;
 }
 
-// The candidates that the walk does not score.  few: the spectrum's, a warp each; else those of the warp that kd_score
-// left, one after another by the whole warp where few of 32 are, side by side otherwise.
-__device__ __forceinline__ void kd_left(const SmemFrag* fp, K2DenseSmem* S, int np, uint32_t q0, int warp, bool few,
-                                            int64_t c0, int64_t c1, const int32_t* c_row, const int8_t* c_maxfz,
-                                            const int64_t* seq_off, const uint8_t* len, const uint64_t* mask,
-                                            const float* mass32, const uint8_t* res, float tol_lo, float tol_hi,
-                                            const K2Out out) {
-  const int lane = threadIdx.x & 31, width = few ? 1 : 32;
-  for (int64_t cw = c0 + warp * width; cw < c1; cw += KD_WARPS * width) {
+// The warp's candidates that kd_score left: one after another by the whole warp where few of 32 are, else side by side.
+__device__ __forceinline__ void kd_left(const SmemFrag* fp, K2DenseSmem* S, int np, uint32_t q0, int warp, int64_t c0,
+                                        int64_t c1, const int32_t* c_row, const int8_t* c_maxfz,
+                                        const int64_t* seq_off, const uint8_t* len, const uint64_t* mask,
+                                        const float* mass32, const uint8_t* res, float tol_lo, float tol_hi,
+                                        const K2Out& out) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t cw = c0 + warp * 32; cw < c1; cw += KD_WARPS * 32) {
     const int64_t c = cw + lane;
-    const bool mine = lane < width && c < c1 && (few || out.lb[c] == KD_LEFT);
+    const bool mine = c < c1 && out.lb[c] == KD_LEFT;
     unsigned todo = __ballot_sync(VK_FULL, mine);
     if (!todo) continue;
     K2Val v{0.f, 0.f, 0.f, 0, 0, 0, 0};
@@ -757,9 +756,8 @@ __device__ __forceinline__ void k2_dense_body(K2DenseSmem& S, const SmemFrag& fp
     RowWords w{};
     kd_begin(w, d, some, res);
     __syncthreads();
-    const bool few = c1 - c0 <= KD_FEW;
-    bool left = few;
-    for (int64_t cw = c0 + warp * 32; cw < c1 && !few; cw += NT) {   // uniform over the warp
+    bool left = false;
+    for (int64_t cw = c0 + warp * 32; cw < c1; cw += NT) {   // uniform over the warp
       const int64_t c = cw + lane;
       left |= kd_score(S, pt, warp, lane, c < c1, d, w, fp, tol_lo, tol_hi, out, c);
       __syncwarp();
@@ -768,8 +766,7 @@ __device__ __forceinline__ void k2_dense_body(K2DenseSmem& S, const SmemFrag& fp
       kd_begin(w, d, more, res);
     }
     if (__any_sync(VK_FULL, left))
-      kd_left(&fp, &S, np, pt.q0, warp, few, c0, c1, c_row, c_maxfz, seq_off, len, mask, mass32, res, tol_lo, tol_hi,
-              out);
+      kd_left(&fp, &S, np, pt.q0, warp, c0, c1, c_row, c_maxfz, seq_off, len, mask, mass32, res, tol_lo, tol_hi, out);
   }
 }
 
