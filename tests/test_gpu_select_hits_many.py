@@ -83,11 +83,11 @@ def _check(specs, counts, topk, closure, copies, n_rows):
     assert bool((s_mt.view(copies, -1) == up(np.bincount(spec, weights=mt, minlength=n_spec), np.int64)).all())
 
 
-# 12 spectra, so 60, 300, 660 and 1,320 of them: lists are left to a CTA from 1,024, 4,096, 16,384 and 65,536 rows
+# 12 spectra, so 60, 660, 1,320 and 4,800 of them: lists are left to a CTA from 1,024, 4,096, 16,384 and 65,536 rows
 @pytest.mark.parametrize("counts", ["small", "equal", "tall", "sparse"])
 @pytest.mark.parametrize("topk,closure", [(1, True), (33, False), (100, True), (256, True), (385, False), (512, False),
                                           (900, False)])
-@pytest.mark.parametrize("copies", [5, 25, 55, 110])
+@pytest.mark.parametrize("copies", [5, 55, 110, 400])
 def test_long_lists_of_many_spectra(counts, topk, closure, copies):
     specs = []
     for n in (511, 513, 640, 1000, 4097):
@@ -101,3 +101,9 @@ def test_long_lists_of_many_spectra(counts, topk, closure, copies):
 @pytest.mark.parametrize("topk,closure", [(40, False), (100, True)])
 def test_more_lists_left_than_ctas(topk, closure):
     _check([[(128, 70128)], [(40, 65580), (100, 130)], [(3, 90)]], "sparse", topk, closure, 400, 71000)
+
+
+@pytest.mark.parametrize("topk,closure", [(40, False), (100, True)])
+def test_several_lists_per_cta(topk, closure):
+    specs = [[(300, 300 + n), (100, 90 + n)] for n in (2100, 2600, 4500)] + [[(3, 90)]]
+    _check(specs, "small", topk, closure, 290, 14000)

@@ -850,9 +850,10 @@ __device__ __forceinline__ bool leave_hits(int64_t hb, int nhs, const int64_t* h
 // big_rows rows or more, leaves the spectrum to select_hits_big_k (n_cand = -1): a CTA has a list done sooner than a
 // warp, but 592 run at once instead of some 2,400, and its last step is one warp's.  Per launch, CTA / warp: 20,000
 // spectra of 603 hits at topk 100 2.86 / 0.39 ms (an eight-pass radix select in global memory took 1.07), 2,000 of
-// 5,070 0.54 / 0.20; 500 of 1,206 0.102 / 0.084, of 5,070 0.135 / 0.187; 32 of 603 0.056 / 0.058, of 1,206 0.062 /
-// 0.082.  Hence big_rows (twice the hits there): 1,024 up to an SM a spectrum, 4,096 up to a CTA each, 16,384 up to two
-// spectra a CTA, else 65,536.
+// 5,070 0.54 / 0.20, of 20,280 0.83 / 0.65; 500 of 1,206 0.102 / 0.084, of 5,070 0.135 / 0.187; 32 of 603 0.056 /
+// 0.058, of 1,206 0.062 / 0.082; and where few of many lists are long, one warp's time is the launch's (777 open
+// windows: 0.051 + 0.178 / 0.134 + 0.177 with those of 4,096 to 16,384 rows).  Hence big_rows (twice the hits above):
+// 1,024 rows up to an SM a spectrum, 4,096 up to two spectra a CTA, 16,384 up to eight, else 65,536.
 // At least 4 CTAs an SM: left to itself the compiler keeps to 56 registers and spills (5% on lists that fit).
 __global__ void __launch_bounds__(TK_WARPS * 32, 4)
 select_hits_k(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
@@ -1473,10 +1474,10 @@ int vk_select_hits(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
   while (list_pow2 < (pair_closure ? 2 : 1) * topk) list_pow2 <<= 1;
   int key_cap = list_pow2 > 512 ? list_pow2 : 512;
   if (key_cap < topk + 128) key_cap *= 2;   // room for new hits beside the topk that stay
-  const int64_t big_rows = n_spec <= HB_FEW       ? 1024      // (see select_hits_k)
-                           : n_spec <= 4 * HB_FEW ? 4096
-                           : n_spec <= 8 * HB_FEW ? 16384
-                                                  : 65536;
+  const int64_t big_rows = n_spec <= HB_FEW        ? 1024      // (see select_hits_k)
+                           : n_spec <= 8 * HB_FEW  ? 4096
+                           : n_spec <= 32 * HB_FEW ? 16384
+                                                   : 65536;
   const size_t per_warp = (size_t)key_cap * 12 + (size_t)list_pow2 * 16 + 1024 + sizeof(HitScratch);
   const size_t sh = per_warp * TK_WARPS;
   if (sh > TK_SMEM) return VK_E_ARG;
