@@ -672,7 +672,7 @@ def _kernel_table(a, p, gi, run, flush, pr, dev):
             K.ptr(gi.partner), p.k1_threshold, p.topk, int(p.pair_closure), cap, K.ptr(tk["h"]), K.ptr(tk["r"]),
             K.ptr(tk["c"]), K.ptr(tk_n), K.ptr(hs_), K.ptr(hm_), K.ptr(ss_), K.ptr(sm_), K.stream()), "select_topk"))
         n_sel = int(((hits["c_cnt"][:n_hit] >= 0)).sum())
-        kern["select_topk_k"] = (ms_tk, n_win * 4 + n_sel * 8 + n_hit * 24 + nh * 12 + n * 16)
+        kern["select_topk_rows_k and select_topk_k"] = (ms_tk, n_win * 4 + n_sel * 8 + n_hit * 24 + nh * 12 + n * 16)
     mlp = None
     if pruned:
         feat = so["feat"]
@@ -709,14 +709,14 @@ def _kernel_table(a, p, gi, run, flush, pr, dev):
     rows = so["c_row"][:n_cand]
     npk = (peaks["off"][1:n + 1] - peaks["off"][:n]).clamp(max=512)
     k2_bytes = int(((21 + gi.length[rows].long() + 5 + 28).sum() + npk.sum() * 8 + n * 16).item())
-    # the path's K2 (thread per candidate after the pruner, warp per spectrum otherwise) and the other for reference
+    # the path's K2 (thread per candidate after the pruner, CTA per spectrum otherwise) and the other for reference
     ms_sp = timed(lambda: K.check(L.vk_k2_spectra(*k2_args, None, *E._k2_ptrs(k2o), K.stream()), "k2_spectra"))
     ms_cd = timed(lambda: K.check(L.vk_k2_cands(*k2_args, *E._k2_ptrs(k2o), K.stream()), "k2_cands"))
     if pruned:
         kern["k2_cands_k"] = (ms_cd, k2_bytes)
-        kern["k2_spectra_k (not used on this path)"] = (ms_sp, k2_bytes)
+        kern["k2_dense_k (not used on this path)"] = (ms_sp, k2_bytes)
     else:
-        kern["k2_spectra_k"] = (ms_sp, k2_bytes)
+        kern["k2_dense_k"] = (ms_sp, k2_bytes)
         kern["k2_cands_k (not used on this path)"] = (ms_cd, k2_bytes)
     if p.search_method == "fused" and not pruned:
         kern = {"fused_search_k": (timed(lambda: E._fused_device(gi, p, 1, peaks, dh, run.n)),

@@ -287,7 +287,8 @@ int vk_k1_hits(const vk_tindex* ix, const vk_frag_params* fp, float tol_lo, floa
  * slots: spectrum s writes n_cand[s] candidates sorted by row at [s*cap, s*cap + n_cand[s]) of c_hyp (i64),
  * c_row (i64), c_cnt (i64); cap >= (pair_closure ? 2 : 1) * topk.  Also hyp_scored (u32, #rows with count > 0)
  * and hyp_matched (u64, sum of counts) per hypothesis, and their sums per spectrum (spec_scored, spec_matched,
- * i64; may be NULL).  cnt holds cnt_cap entries: a window whose slice would end past it counts as empty. */
+ * i64; may be NULL).  cnt holds cnt_cap entries: a window whose slice would end past it counts as empty.  One launch
+ * or, at 1 <= thr <= 254 and topk <= 512, two: the spectra whose windows are pairwise disjoint, then those left. */
 int vk_select_topk(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
                    const int64_t* win_off, const int32_t* cnt, int64_t cnt_cap, const int64_t* partner, int thr,
                    int topk, int pair_closure, int cap, int64_t* c_hyp, int64_t* c_row, int64_t* c_cnt, int64_t* n_cand,
@@ -303,7 +304,9 @@ int vk_select_topk(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo,
  * seg_cnt locate each hypothesis' hit segments (per 32 segments, one parallel read of their counts, then one of
  * their hits).  The same candidates as vk_select_topk over vk_k1_tiles' dense counts with
  * thr = vk_k1_hits' thr.  Without closure, when a spectrum's windows are pairwise disjoint (the usual case), the
- * hits are collected in row order and kept in that order, with no sort. */
+ * hits are collected in row order and kept in that order, with no sort.  A warp per spectrum; a second launch (none
+ * at topk <= 32 without closure) gives a CTA to each list that is more than a warp holds and comes from long
+ * windows. */
 int vk_select_hits(int n_spec, const int64_t* spec_hyp_off, const int64_t* h_lo, const int64_t* h_hi,
                    const int64_t* win_off, const int8_t* hyp_shift, const uint32_t* seg_cnt, const uint64_t* hit_rc,
                    const uint32_t* hit_isum,
@@ -323,10 +326,10 @@ int vk_compact_hits(int n_spec, int cap, const int64_t* n_cand, const int64_t* c
                     uint32_t* c_isum, void* stream);
 
 /* K2 exact rescoring (reference kernels.cu:263-376), B200 launch: a CTA per spectrum at a time (one warp with
- * c_shift), lanes over candidates, the spectrum's (first 512) peaks in shared memory.  Candidates of spectrum s are [cand_off[s], cand_off[s+1])
- * (cand_off has n_spec+1 entries, spectrum ids are 0..n_spec-1).  c_shift NULL: the closed mode; else the
- * per-candidate precursor shift (Da, f32) of the open / mass-offset modes: shifted and unshifted ions scored as
- * the reference's shift mode (kernels.cu:294-363). */
+ * c_shift), lanes over candidates, the spectrum's (first 512) peaks in shared memory.  Candidates of spectrum s are
+ * [cand_off[s], cand_off[s+1]) (cand_off has n_spec+1 entries, spectrum ids are 0..n_spec-1).  c_shift NULL: the
+ * closed mode; else the per-candidate precursor shift (Da, f32) of the open / mass-offset modes: shifted and unshifted
+ * ions scored as the reference's shift mode (kernels.cu:294-363). */
 int vk_k2_spectra(const vk_frag_params* fp, int n_spec, const int64_t* cand_off, const int32_t* c_row,
                   const int8_t* c_maxfz, const int64_t* pk_off, const float* pk_mass, const float* pk_int,
                   const int64_t* seq_off, const uint8_t* len, const uint64_t* mask, const float* mass32,
